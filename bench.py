@@ -250,7 +250,7 @@ class Clocks:
 def pw_kernel_name(variant, window):
     """Name of the plane-wave fused kernel a plan's variant launches."""
     if variant == 9:
-        return "pw_tc_kernel<%s> (mma.sync m16n8k16, fp16 hi/lo operands)" % window
+        return "pw_tc_kernel (tcgen05, fp16 hi/lo operands; window %s from the plan's table)" % window
     shapes = {1: (1, 11), 2: (2, 4), 3: (2, 2), 4: (4, 1)}
     ept, na = shapes[(variant - 1) % 4 + 1]
     return "%s<%d,%d,%s>" % ("pw_event_kernel" if variant <= 4 else "pw_fused_kernel", ept, na, window)
@@ -434,15 +434,16 @@ def run_ours(args):
             "peak_source": "measured FP32 FMA throughput (fnum_diag_fp32_peak); MEASURED_PEAKS.json "
             "holds only HBM and bf16 figures"}
     if args.kernel == "fused" and info["kernel_variant"] == 9:
-        # the tensor pipe: three m16n8k16 products per 16 voxels x 8 elements x 4 angles
-        mpeak = _lib.C.c_double(0.0)
-        _lib.check(_lib.lib().fnum_diag_mma_f16_peak(local, _lib.C.byref(mpeak)))
-        na_pass = min(12, len(wl.angles))
-        mma_flops = info["executed_terms"] / (16.0 * 8.0 * na_pass) * 3 * 3 * 2 * 16 * 8 * 16  # 3 n-tiles
-        roof["tensor"] = {"achieved": mma_flops / (bf_avg_ms * 1e-3) / 1e12, "peak": mpeak.value,
-                          "unit": "TFLOP/s", "frac": mma_flops / (bf_avg_ms * 1e-3) / 1e12 / mpeak.value,
-                          "work": "mma.sync m16n8k16 instructions issued (3 fp16 products per operand tile)",
-                          "peak_source": "measured mma.sync m16n8k16 f16/f32 throughput (fnum_diag_mma_f16_peak)"}
+        # the tensor pipe: three products of 128 voxels x 8 complex elements x n columns per bin
+        na = len(wl.angles)
+        n = 16 if na <= 8 else (32 if na <= 16 else (48 if na <= 24 else 64))
+        passes = -(-na // (n // 2 if n > 16 else 8))
+        mma_flops = info["executed_terms"] / na * passes * 3 * 2.0 * 2 * n
+        mpeak = measured_peaks().get("bf16_tflops")
+        roof["tensor"] = {"achieved": mma_flops / (bf_avg_ms * 1e-3) / 1e12, "peak": mpeak,
+                          "unit": "TFLOP/s", "frac": mma_flops / (bf_avg_ms * 1e-3) / 1e12 / mpeak if mpeak else None,
+                          "work": "tcgen05.mma instructions issued (3 fp16 products per operand tile)",
+                          "peak_source": "MEASURED_PEAKS.json (cuBLAS bf16 burst)"}
     if rank != 0:
         return
     acc = accuracy_of(wl, win, fn, img[0].cpu().numpy())
@@ -464,7 +465,7 @@ def run_ours(args):
            "stage_ms": {"band_dft": float(np.mean(dft_ms)), "beamform": bf_avg_ms},
            "e2e": e2e, "roofline": roof, "cpu_baseline": cb, "clocks": clk, "accuracy": acc,
            # per step: the band DFT (operand split + tcgen05 GEMM) and the beamformer, which adds
-           # the scale and fragment kernels for variant 9; no library kernels
+           # the scale and operand kernels for variant 9; no library kernels
            "gpu_launches": args.steps * (5 if (args.kernel == "fused" and info["kernel_variant"] == 9) else 3),
            "library_launches": {}}
     if anchor is not None:
@@ -694,11 +695,11 @@ def run_batch(args):
                           "sum_of_standalone": float(np.sum(solo))},
            "clocks": clk,
            # per frame: the band DFT (two kernels); a compounded tensor-core frame then its
-           # scale and fragment kernels, its tiles beamformed by the persistent launches (one
-           # per window and pass width); any other frame per beamform launch the kernel (+
-           # scale and fragment kernels for the tensor-core variant)
+           # scale and operand kernels, its tiles beamformed by the persistent launches (one
+           # per class of angle counts); other tensor-core frames add their own launch, FP32
+           # frames one per image
            "gpu_launches": args.steps * (n_persist_launches + sum(
-               2 + (2 if (p.n_out == 1 and v == 9) else (1 if p.n_out == 1 else p.n_angles) * (3 if v == 9 else 1))
+               2 + ((2 if p.n_out == 1 else 3) if v == 9 else (1 if p.n_out == 1 else p.n_angles))
                for p, v in zip(plans, variants)))}
     print(json.dumps(out))
     batch.close()

@@ -20,7 +20,7 @@ EXPORTS = (
     "fnum_batch_frame_times", "fnum_batch_destroy", "fnum_pw_plan_set_sound_speed", "fnum_pw_sharpness_grad",
     "fnum_plan_m_signal", "fnum_plan_set_kernel_variant", "fnum_diag_mma_f16_peak", "fnum_host_cache_info",
     "fnum_plan_spectra", "fnum_pw_adjoint", "fnum_plan_set_spectra", "fnum_das_pw_sharpness_grad",
-    "fnum_batch_info", "fnum_plan_set_shape",
+    "fnum_batch_info", "fnum_plan_set_shape", "fnum_pw_forward",
 )
 
 ABI_VERSION = 4   # FNUM_ABI_VERSION of include/fnum.h
@@ -196,6 +196,8 @@ def lib():
     L.fnum_das_pw_sharpness_grad.argtypes = [C.POINTER(PWDesc), _dp, C.c_int, _dp, _dp, _dp, _fp, _fp]
     L.fnum_pw_adjoint.restype = C.c_int
     L.fnum_pw_adjoint.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, _dp, C.c_void_p]
+    L.fnum_pw_forward.restype = C.c_int
+    L.fnum_pw_forward.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
     L.fnum_plan_set_spectra.restype = C.c_int
     L.fnum_plan_set_spectra.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
     L.fnum_plan_spectra.restype = C.c_int

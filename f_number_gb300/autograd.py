@@ -5,7 +5,7 @@ speed of sound c.
     image = pw_beamform(plan, X, c)       # complex64 [N_x, N_z] on the plan's GPU
 
 The forward is fnum_plan_set_spectra + fnum_pw_plan_set_sound_speed +
-fnum_plan_execute_beamform (the fused kernels); the backward is fnum_pw_adjoint
+fnum_pw_forward (the fused kernels); the backward is fnum_pw_adjoint
 (the hand-written adjoint kernel).  As in fnum_pw_sharpness_grad, the DFT order,
 band, F table and apertures are those of the speed the plan was created with;
 only the phases follow c.  The reference (das_pw.m, +cuda/gpu_bf_das_pw_rf.cu)
@@ -34,7 +34,7 @@ class PWBeamform(torch.autograd.Function):
         plan.set_sound_speed(c_val)
         plan.set_spectra(spectra)
         img = torch.empty((1, plan.n_x, plan.n_z), dtype=torch.complex64, device=spectra.device)
-        plan.execute_beamform(img)
+        plan.forward(img)
         ctx.plan = plan
         ctx.c = c_val
         ctx.c_is_tensor = torch.is_tensor(c)

@@ -358,6 +358,20 @@ __device__ __forceinline__ int sa_seg_find(const int4* seg, int nseg, int kt) {
   return lo;
 }
 
+// splits two FP32 values into packed fp16 hi and lo = fp16(x - hi), the residual from
+// sm_100's mixed-precision FMA: one instruction per value (fp16 source, fp32 result)
+__device__ __forceinline__ void tc_split_mx(float x0, float x1, unsigned& hi, unsigned& lo) {
+  asm("{\n\t.reg .b16 h0, h1, m;\n\t.reg .f32 l0, l1;\n\t"
+      "cvt.rn.f16x2.f32 %0, %3, %2;\n\t"
+      "mov.b32 {h0, h1}, %0;\n\t"
+      "mov.b16 m, 0xBC00;\n\t"
+      "fma.rn.f32.f16 l0, h0, m, %2;\n\t"
+      "fma.rn.f32.f16 l1, h1, m, %3;\n\t"
+      "cvt.rn.f16x2.f32 %1, l1, l0;\n\t}"
+      : "=&r"(hi), "=r"(lo)
+      : "f"(x0), "f"(x1));
+}
+
 // power-of-two scale that brings the spectra below 2^14 (exact in both directions)
 __device__ __forceinline__ float tc_scale(unsigned maxbits) {
   const float m = __uint_as_float(maxbits);

@@ -624,6 +624,55 @@ int setup_tc_dft(fnum_plan* P, int nsig, int k_lb, int K) {
   return e == cudaSuccess ? FNUM_OK : cuda_status(e);
 }
 
+// blocks of a plane-wave plan's current kernel; the recurrence kernels' segment scratch
+// holds max_grid blocks
+int pw_grid(const fnum_plan* P) {
+  const int g = fnum::pw_fused_grid(P->pw, nullptr);
+  return fnum::pw_variant_of(P->pw) == fnum::TC_VARIANT ? g : std::min(g, P->max_grid);
+}
+
+// Tensor-core plane-wave kernel: window table, operand tiles and scratch.
+int setup_pw_tc(fnum_plan* P, int na, int n_img) {
+  fnum::PWDev& D = P->pw;
+  const int ne = D.ne;
+  D.ne_pad = (ne + 15) / 16 * 16;
+  // the table covers all columns, or as many as fit 512 MB (then it is refilled per launch)
+  const size_t col = (size_t)(ne + 1) * D.ne_pad;
+  const size_t fit = std::max<size_t>((((size_t)512 << 20) / (col * sizeof(float))) / 4 * 4, 4);
+  D.wt_c0 = 0;
+  D.wt_nc = (int)std::min<size_t>(fit, D.nx);
+  fnum::pw_tc_pick_split(D);
+  const size_t tiles = (size_t)((D.nx + fnum::TILE_X - 1) / fnum::TILE_X) * ((D.nz + fnum::TILE_Z - 1) / fnum::TILE_Z);
+  // the mma.sync kernels read the same buffer as fragments (32 uint4 per n-tile, bin and group of
+  // 8 elements; the derivative kernel in passes of 12 angles)
+  D.tc_S = (ne + 7) / 8 + fnum::TC_KS - 1;
+  D.tc_nt = fnum::tc_ntiles_for(na);
+  size_t n_b = fnum::pw_tc_operand_bytes(na, D.K, D.ne_pad);
+  for (int nt : {3, D.tc_nt})
+    n_b = std::max(n_b, (size_t)((na + 4 * nt - 1) / (4 * nt)) * D.K * D.tc_S * 32 * nt * sizeof(uint4));
+  const size_t n_u = fnum::pw_tc_scratch_bytes(fnum::pw_tc_grid(D));
+  const size_t n_part = D.split > 1 ? (size_t)D.split * n_img * D.nx * D.nz : 0;
+  // one allocation for all of it
+  const size_t sizes[] = {col * D.wt_nc * sizeof(float), (size_t)(ne + 1) * D.wt_nc * sizeof(float), n_b, n_u,
+                          n_part * sizeof(float2), tiles * sizeof(unsigned), sizeof(unsigned)};
+  size_t off[8] = {0};
+  for (int i = 0; i < 7; ++i) off[i + 1] = off[i] + (sizes[i] + 255) / 256 * 256;
+  unsigned char* m = nullptr;
+  if (const int s = P->alloc(&m, off[7])) return s;
+  float* tab = (float*)m;
+  float* sum = (float*)(m + off[1]);
+  D.w_tab = tab;
+  D.w_sum = sum;
+  D.tc_B = (uint4*)(m + off[2]);
+  D.u_scr = (float4*)(m + off[3]);
+  D.part = (float2*)(m + off[4]);
+  D.tile_cnt = (unsigned*)(m + off[5]);
+  D.tc_max = (unsigned*)(m + off[6]);
+  P->info.scratch_bytes += (long long)off[7];
+  if (D.wt_nc == D.nx) FNUM_CUDA(fnum::launch_pw_tc_window(D, tab, sum, 0));
+  return FNUM_OK;
+}
+
 int make_pw_plan(const fnum_pw_desc* d, const double* angles, int na, int flags, fnum_plan** out) {
   int s = check_pw(d, angles, na);
   if (s) return s;
@@ -676,6 +725,9 @@ int make_pw_plan(const fnum_pw_desc* d, const double* angles, int na, int flags,
     txf[a] = make_float4((float)ex, (float)ez, (float)xref, 0.0f);
   }
   g_table(P->F, gg);
+  D.gmax = gg[0];   // the widest aperture of the band: F <= FLT_EPSILON (marked), else the largest 1 / (2 F)
+  for (const dfl& v : gg)
+    if (v.x < 0.0f || (D.gmax.x >= 0.0f && (double)v.x + v.y > (double)D.gmax.x + D.gmax.y)) D.gmax = v;
   std::vector<float> Ff(b.K);
   for (int i = 0; i < b.K; ++i) Ff[i] = (float)P->F[i];
   dfl* p;
@@ -747,19 +799,9 @@ int make_pw_plan(const fnum_pw_desc* d, const double* angles, int na, int flags,
     D.seg = seg;
     P->info.scratch_bytes =
         (long long)P->max_grid * fnum::NTHREADS * D.seg_cap * fnum::PW_SEG_INT4 * (long long)sizeof(int4);
-    // tensor-core variant: spectra as mma fragments (32 uint4 per n-tile, bin and group of 8 elements)
-    D.tc_S = (ne + 7) / 8 + fnum::TC_KS - 1;   // a pass may start in the last group of 8
-    D.tc_nt = fnum::tc_ntiles_for(na);
-    // the fragments in the layout of the plan's passes, or of 12-angle passes (the
-    // derivative kernel's), whichever is larger
-    size_t n_tc = 0;
-    for (int nt : {3, D.tc_nt})
-      n_tc = std::max(n_tc, (size_t)((na + 4 * nt - 1) / (4 * nt)) * D.K * D.tc_S * 32 * nt);
-    if ((s = P->alloc(&D.tc_B, n_tc))) goto fail;
-    if ((s = P->alloc(&D.tc_max, 1))) goto fail;
-    P->info.scratch_bytes += (long long)(n_tc * sizeof(uint4) + sizeof(unsigned));
+    if ((s = setup_pw_tc(P, na, (flags & FNUM_FLAG_COMPOUND) ? 1 : na))) goto fail;
     // the default variant may now be the tensor-core one
-    P->grid = std::min(fnum::pw_fused_grid(D, &bps), P->max_grid);
+    P->grid = pw_grid(P);
   }
   {
     cudaError_t e = fnum::launch_twiddles(P->tw, b.N, 0);
@@ -972,6 +1014,8 @@ int plan_beamform(fnum_plan* P, void* image, float* w, float* w2, cudaStream_t s
                           : fnum::launch_pw_fused(D, P->grid, (float2*)image, w, st);
     return cuda_status(e);
   }
+  if (!plain && fnum::pw_variant_of(D) == fnum::TC_VARIANT)   // all angles in one launch
+    return cuda_status(fnum::launch_pw_tc(D, true, (float2*)image, w, st));
   for (int a = 0; a < D.na; ++a) {
     fnum::PWDev Da = D;
     Da.na = 1;
@@ -1384,7 +1428,7 @@ int fnum_plan_set_kernel_variant(fnum_plan* plan, int variant) {
   if (plan->pw.m_sem) return variant == 0 ? FNUM_OK : FNUM_ERR_ARGUMENT;     // one per-term kernel
   FNUM_CUDA(cudaSetDevice(plan->device));
   plan->pw.variant = variant;
-  plan->grid = std::min(fnum::pw_fused_grid(plan->pw, nullptr), plan->max_grid);
+  plan->grid = pw_grid(plan);
   return FNUM_OK;
 }
 
@@ -1457,7 +1501,7 @@ int fnum_plan_autotune(fnum_plan* plan, const void* d_rf, int rf_is_double, int*
   int best_g = plan->grid;
   // times the plan's current variant and shape (a warm-up, then two beamforms)
   auto trial = [&]() -> int {
-    plan->grid = std::min(fnum::pw_fused_grid(plan->pw, nullptr), plan->max_grid);
+    plan->grid = pw_grid(plan);
     int st2 = plan_beamform(plan, img, nullptr, nullptr, st);
     if (st2) return st2;
     float t = 0.0f;
@@ -1546,7 +1590,7 @@ int fnum_plan_set_shape(fnum_plan* plan, int blocks_per_sm, int bin_chunk) {
     D.flush_chunks = bin_chunk == 128 ? 2 : 4;
   }
   D.blocks_per_sm = blocks_per_sm;
-  plan->grid = std::min(fnum::pw_fused_grid(D, nullptr), plan->max_grid);
+  plan->grid = pw_grid(plan);
   return FNUM_OK;
 }
 
@@ -1557,10 +1601,10 @@ struct fnum_batch {
   cudaGraphExec_t exec = nullptr;
   cudaEvent_t start = nullptr;
   std::vector<cudaEvent_t> done;   // per frame, recorded when the frame's image is complete
-  // persistent tensor-core launches, one per window and pass width of the compounded tensor-core frames
+  // persistent tensor-core launches, one per class (pw_tc_class) of the compounded tensor-core frames
   struct TcGroup {
-    int window_id = 0, grid = 0;
-    int nt = 3;                     // n-tiles per angle pass of the group's frames
+    int cls = 0, grid = 0;
+    int widest = 1;                 // largest angle count of the group's frames
     std::vector<int> frames;        // batch frame indices, largest first
     fnum::PWBatchDev dev{};
   };
@@ -1584,7 +1628,7 @@ namespace {
 // whose kernel variant is the tensor-core one
 bool tc_persistent(const fnum_plan* P) {
   return P->kind == 0 && P->n_out == 1 && !P->pw.m_sem && !(P->flags & FNUM_FLAG_PLAIN_KERNEL) &&
-         fnum::pw_variant_of(P->pw) == fnum::TC_VARIANT && P->pw.tc_B;
+         fnum::pw_variant_of(P->pw) == fnum::TC_VARIANT && P->pw.tc_B && P->pw.wt_nc == P->pw.nx;
 }
 
 template <typename T>
@@ -1601,29 +1645,24 @@ int batch_upload(fnum_batch* B, T** dst, const std::vector<T>& v) {
   return FNUM_OK;
 }
 
-// descriptor arrays, tile prefix sums, counter and segment scratch of one persistent group
+// descriptor arrays, item prefix sums, counter and scratch of one persistent group
 int build_tc_group(fnum_batch* B, fnum_batch::TcGroup& G, fnum_plan* const* plans, void* const* d_images,
                    float* const* d_weights) {
   std::vector<fnum::PWDev> frames;
   std::vector<float2*> images;
   std::vector<float*> weights;
   std::vector<int> tile_start(1, 0);
-  int max_ne = 1, seg_cap = 1;
   for (int f : G.frames) {
     const fnum::PWDev& D = plans[f]->pw;
     frames.push_back(D);
     images.push_back((float2*)d_images[f]);
     weights.push_back(d_weights ? d_weights[f] : nullptr);
-    tile_start.push_back(tile_start.back() + fnum::pw_tc_tiles(D));
-    max_ne = std::max(max_ne, D.ne);
-    seg_cap = std::max(seg_cap, D.seg_cap);
+    tile_start.push_back(tile_start.back() + fnum::pw_tc_items(D));
   }
   int s;
   fnum::PWBatchDev& dev = G.dev;
   dev.n_frames = (int)G.frames.size();
-  dev.max_ne = max_ne;
-  dev.seg_cap = seg_cap;
-  G.grid = fnum::pw_tc_batch_grid(max_ne, G.window_id, G.nt, nullptr);
+  G.grid = std::min(fnum::pw_tc_batch_grid(), tile_start.back());
   fnum::PWDev* d_frames = nullptr;
   float2** d_img = nullptr;
   float** d_w = nullptr;
@@ -1634,25 +1673,19 @@ int build_tc_group(fnum_batch* B, fnum_batch::TcGroup& G, fnum_plan* const* plan
       (s = batch_upload(B, &d_w, weights)) || (s = batch_upload(B, &d_ts, tile_start)) ||
       (s = batch_upload(B, &d_counter, zero)))
     return s;
-  void* seg = nullptr;
-  cudaError_t e = cudaMalloc(&seg, (size_t)G.grid * fnum::NTHREADS * seg_cap * fnum::PW_SEG_INT4 * sizeof(int4));
+  void* u = nullptr;
+  cudaError_t e = cudaMalloc(&u, fnum::pw_tc_scratch_bytes(G.grid));
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     return cuda_status(e);
   }
-  B->allocs.push_back(seg);
-  // the descriptors the kernel reads carry the batch's segment scratch
-  for (auto& D : frames) {
-    D.seg = (int4*)seg;
-    D.seg_cap = seg_cap;
-  }
-  FNUM_CUDA(cudaMemcpy(d_frames, frames.data(), frames.size() * sizeof(fnum::PWDev), cudaMemcpyHostToDevice));
+  B->allocs.push_back(u);
   dev.frames = d_frames;
   dev.images = d_img;
   dev.weights = d_w;
   dev.tile_start = d_ts;
   dev.counter = d_counter;
-  dev.seg = (int4*)seg;
+  dev.u_scr = (float4*)u;
   return FNUM_OK;
 }
 
@@ -1690,20 +1723,20 @@ int fnum_batch_create(fnum_plan* const* plans, int n, const void* const* d_rf, c
   for (int i = 0; i < n && e == cudaSuccess; ++i) e = cudaEventCreate(&B->done[i]);
   for (int i = 0; i < k && e == cudaSuccess; ++i) e = cudaStreamCreateWithFlags(&st[i], cudaStreamNonBlocking);
   for (int i = 0; i < k && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&fj[i], cudaEventDisableTiming);
-  // compounded tensor-core frames go to persistent launches (one per window and pass width), the others
+  // compounded tensor-core frames go to persistent launches (one per class), the others
   // keep a launch per frame on the branches
   std::vector<char> persistent(n, 0);
   for (int f : order) {
     if (!tc_persistent(plans[f])) continue;
     persistent[f] = 1;
-    const int w = plans[f]->pw.window_id, nt = plans[f]->pw.tc_nt == 4 ? 4 : 3;
+    const int cls = fnum::pw_tc_class(plans[f]->pw.na);
     size_t gi = 0;
-    while (gi < B->groups.size() && (B->groups[gi].window_id != w || B->groups[gi].nt != nt)) ++gi;
+    while (gi < B->groups.size() && B->groups[gi].cls != cls) ++gi;
     if (gi == B->groups.size()) {
       B->groups.emplace_back();
-      B->groups.back().window_id = w;
-      B->groups.back().nt = nt;
+      B->groups.back().cls = cls;
     }
+    B->groups[gi].widest = std::max(B->groups[gi].widest, plans[f]->pw.na);
     B->groups[gi].frames.push_back(f);   // `order` is largest first
     ++B->persistent_frames;
   }
@@ -1738,7 +1771,10 @@ int fnum_batch_create(fnum_plan* const* plans, int n, const void* const* d_rf, c
       cudaStream_t q = st[rr++ % k];
       if ((s = plan_dft(plans[f], d_rf[f], rf_is_double ? rf_is_double[f] : 0, q))) break;
       e = cudaMemsetAsync(plans[f]->counters, 0, 5 * sizeof(unsigned long long), q);
-      if (e == cudaSuccess) e = fnum::launch_pw_tc_prep(plans[f]->pw, q);
+      int widest = 1;
+      for (const auto& G : B->groups)
+        if (G.cls == fnum::pw_tc_class(plans[f]->pw.na)) widest = G.widest;
+      if (e == cudaSuccess) e = fnum::launch_pw_tc_operand(plans[f]->pw, widest, q);
       if (e != cudaSuccess) s = cuda_status(e);
     }
     for (int i = 1; i < k && !s; ++i) {
@@ -1748,7 +1784,7 @@ int fnum_batch_create(fnum_plan* const* plans, int n, const void* const* d_rf, c
     }
     for (auto& G : B->groups) {
       if (s) break;
-      e = fnum::launch_pw_tc_batch(G.dev, G.window_id, G.nt, G.grid, st[0]);
+      e = fnum::launch_pw_tc_batch(G.dev, G.widest, G.grid, st[0]);
       for (size_t j = 0; j < G.frames.size() && e == cudaSuccess; ++j)
         e = cudaEventRecordWithFlags(B->done[G.frames[j]], st[0], cudaEventRecordExternal);
       if (e != cudaSuccess) s = cuda_status(e);
@@ -1886,12 +1922,13 @@ int adjoint_buffers(fnum_plan* plan, cudaStream_t st) {
 
 // dL/dX* into gX and (if dloss_dc) dL/dc for the cotangent G = dL/dI*, on the plan's
 // spectra.  dL/dc needs the derivative image adj_D of those spectra: have_D says that the
-// caller has just computed it (launch_pw_tc_deriv), else it is computed here.
+// caller has just computed it, else it is computed here (launch_pw_mma_deriv, whose
+// rounding goes with fnum_pw_forward's).
 int adjoint_core(fnum_plan* plan, const float2* G, float2* gX, double* dloss_dc, bool have_D, cudaStream_t st) {
   fnum::PWDev& D = plan->pw;
   const long long nvox = (long long)D.nx * D.nz;
   if (dloss_dc) {
-    if (!have_D) FNUM_CUDA(fnum::launch_pw_tc_deriv(D, plan->adj_img, plan->adj_D, st));
+    if (!have_D) FNUM_CUDA(fnum::launch_pw_mma_deriv(D, plan->max_grid, plan->adj_img, plan->adj_D, st));
     FNUM_CUDA(fnum::launch_pw_dc_reduce(G, plan->adj_D, nvox, 4.0 * M_PI / plan->c, plan->adj_sums + 2, st));
   }
   if (gX) FNUM_CUDA(fnum::launch_pw_adjoint(D, G, plan->adj_invw, plan->adj_gmax, gX, plan->adj_acc, st));
@@ -1917,6 +1954,21 @@ int fnum_plan_set_spectra(fnum_plan* plan, const void* d_spectra, void* stream) 
   return FNUM_OK;
 }
 
+int fnum_pw_forward(fnum_plan* plan, void* d_image, void* stream) {
+  if (!plan || !d_image || plan->kind != 0 || plan->n_out != 1) return FNUM_ERR_ARGUMENT;
+  FNUM_CUDA(cudaSetDevice(plan->device));
+  cudaStream_t st = (cudaStream_t)stream;
+  if (plan->pw.m_sem || (plan->flags & FNUM_FLAG_PLAIN_KERNEL) != 0)
+    return fnum::plan_beamform(plan, d_image, nullptr, nullptr, st);
+  FNUM_CUDA(cudaMemsetAsync(plan->counters, 0, 5 * sizeof(unsigned long long), st));
+  fnum::PWDev D = plan->pw;
+  D.variant = fnum::pw_mma_variant_of(D);
+  if (D.variant == fnum::TC_VARIANT)
+    return fnum::cuda_status(fnum::launch_pw_mma(D, plan->max_grid, (float2*)d_image, st));
+  const int grid = std::min(fnum::pw_fused_grid(D, nullptr), plan->max_grid);
+  return fnum::cuda_status(fnum::launch_pw_fused(D, grid, (float2*)d_image, nullptr, st));
+}
+
 int fnum_pw_adjoint(fnum_plan* plan, const void* d_cotangent, void* d_grad_spectra, double* dloss_dc, void* stream) {
   if (!plan || !d_cotangent || plan->kind != 0 || plan->n_out != 1 || plan->pw.m_sem) return FNUM_ERR_ARGUMENT;
   FNUM_CUDA(cudaSetDevice(plan->device));
@@ -1939,7 +1991,7 @@ int fnum_pw_sharpness_grad(fnum_plan* plan, const void* d_rf, int rf_is_double, 
   if ((s = fnum::adjoint_buffers(plan, st))) return s;
   if ((s = plan_dft(plan, d_rf, rf_is_double, st))) return s;
   // the image and its derivative in c in one pass of the tensor-core kernel
-  FNUM_CUDA(fnum::launch_pw_tc_deriv(D, plan->adj_img, plan->adj_D, st));
+  FNUM_CUDA(fnum::launch_pw_mma_deriv(D, plan->max_grid, plan->adj_img, plan->adj_D, st));
   FNUM_CUDA(fnum::launch_pw_sharp_sums(plan->adj_img, nvox, plan->adj_sums, st));
   double S[2] = {0.0, 0.0};
   FNUM_CUDA(cudaMemcpyAsync(S, plan->adj_sums, sizeof(S), cudaMemcpyDeviceToHost, st));

@@ -18,12 +18,11 @@ constexpr int TILE_Z = 32;
 constexpr int NTHREADS = TILE_X * TILE_Z;
 // band bins per shared-memory spectrum chunk; flushes happen on chunk edges
 constexpr int KCHUNK = 64;
-// tensor-core plane-wave kernel: 4 warps of 16 voxels, TC_TILE_X columns x TILE_Z rows
+// mma.sync plane-wave kernel: 4 warps of 16 voxels, TC_TILE_X columns x TILE_Z rows
 constexpr int TC_TILE_X = 2;
 constexpr int TC_NA = 12;   // angles per angle pass (3 mma n-tiles of 4 complex angles)
-// A plane-wave plan's tensor-core kernel runs passes of 3 n-tiles (12 angles) or, when
-// that takes fewer passes (13-16, 25-32, 37-64 angles, ...), of 4 (16 angles): each pass
-// forms the same A operands, so fewer passes is less work.
+// its passes hold 3 n-tiles (12 angles) or, where that takes fewer passes (13-16, 25-32,
+// 37-64 angles, ...), 4 (16 angles): each pass forms the same A operands
 inline int tc_ntiles_for(int na) { return ((na + 15) / 16 < (na + TC_NA - 1) / TC_NA) ? 4 : 3; }
 constexpr int TC_EP = 16;   // elements per pass: TC_KS mma k-steps of 8 complex elements
 constexpr int TC_KS = TC_EP / 8;
@@ -74,12 +73,25 @@ struct PWDev {
   int x_na, x_a0;
   // scratch: [grid][NTHREADS][seg_cap] int4
   int4* seg;
-  // tensor-core variant: spectra as mma B fragments [angle pass][K][tc_S][3][32] (uint4),
-  // and the largest |component| of the spectra (float bits) that sets their fp16 scale
+  // tensor-core variant: spectra as B tiles of the products (pw_tc_operand_kernel; the mma.sync
+  // kernel's fragments [angle pass][K][tc_S][tc_nt][32] share the buffer), and the largest
+  // |component| of the spectra (float bits) that sets their fp16 scale
   uint4* tc_B;
   unsigned* tc_max;
-  int tc_S;            // element groups of 8 in tc_B (TC_KS - 1 zero groups of padding included)
-  int tc_nt;           // mma n-tiles per angle pass of the tensor-core kernel (3 or 4; 0 reads as 3)
+  int tc_S;            // element groups of 8 in the fragments (TC_KS - 1 zero groups of padding included)
+  int tc_nt;           // mma n-tiles per angle pass (3 or 4)
+  // tensor-core kernel (fnum_pw_tc.cu): window table of columns wt_c0 .. wt_c0 + wt_nc - 1
+  // [column][ne + 1][ne_pad] and its row sums, the band's largest aperture, receive delays
+  // of the resident blocks, and for a band split into `split` ranges of split_bins bins
+  // their partial images and the finished ranges per tile
+  const float* w_tab;
+  const float* w_sum;
+  int ne_pad, wt_c0, wt_nc;
+  dfl gmax;
+  float4* u_scr;
+  int split, split_bins;
+  float2* part;
+  unsigned* tile_cnt;
   unsigned long long* counters;   // [0] active terms, [1] zero-weight bins, [2] error bits,
                                   // [3] tile counter, [4] executed recurrence steps
   // the per-voxel FP32 kernel reads the reference's float geometry
@@ -130,16 +142,16 @@ struct SADev {
 
 // One persistent launch of the tensor-core beamformer over the tiles of many
 // compounded frames (fnum_batch_*): per-frame descriptors and outputs in device
-// memory, the tiles numbered frame after frame (tile_start holds the prefix sums),
-// one tile counter and one segment scratch for the launch.
+// memory, the items (a tile and a range of its bins) numbered frame after frame (tile_start holds the prefix sums),
+// one item counter and one scratch for the launch.
 struct PWBatchDev {
   const PWDev* frames;       // [n_frames]
   float2* const* images;     // [n_frames] image of each frame
   float* const* weights;     // [n_frames] weights of each frame (entries may be null)
   const int* tile_start;     // [n_frames + 1]
-  int n_frames, max_ne, seg_cap;
+  int n_frames;
   unsigned long long* counter;
-  int4* seg;                 // [grid][NTHREADS][seg_cap]
+  float4* u_scr;             // receive delays of the resident blocks
 };
 
 // error bits in counters[2] (beamformers) and counters[5] (band DFT)
@@ -200,16 +212,27 @@ int pw_variant_of(const PWDev& d);
 int sa_fused_grid(const SADev& d, int* blocks_per_sm);
 cudaError_t launch_pw_fused(const PWDev& d, int grid, float2* image, float* weights, cudaStream_t s);
 // the compounded image and, in dimage, Draw with dI/dc = -(2 pi i / c) Draw (tensor cores;
-// prepares the fragments itself)
-cudaError_t launch_pw_tc_deriv(const PWDev& d, float2* image, float2* dimage, cudaStream_t s);
-// the tensor-core variant's spectra scale and B fragments for frame d (before a batch launch),
-// laid out for passes of nt n-tiles (0: the plan's own, d.tc_nt)
-cudaError_t launch_pw_tc_prep(const PWDev& d, cudaStream_t s, int nt = 0);
-// tiles of a frame for the tensor-core kernel; grid of the batch kernel with all blocks resident
-int pw_tc_tiles(const PWDev& d);
-// nt: the n-tiles per angle pass of every frame of the launch (frames are grouped by it)
-int pw_tc_batch_grid(int max_ne, int window_id, int nt, int* blocks_per_sm);
-cudaError_t launch_pw_tc_batch(const PWBatchDev& B, int window_id, int nt, int grid, cudaStream_t s);
+// prepares the operand tiles itself)
+cudaError_t launch_pw_mma_deriv(const PWDev& d, int max_grid, float2* image, float2* dimage, cudaStream_t s);
+// the image from mma.sync (max_grid: blocks that the segment scratch holds)
+cudaError_t launch_pw_mma(const PWDev& d, int max_grid, float2* image, cudaStream_t s);
+int pw_mma_variant_of(const PWDev& d);   // the variant of the differentiable forward pass (9: launch_pw_mma)
+// --- plane wave on the tensor cores (fnum_pw_tc.cu) -------------------------
+int pw_tc_class(int na);       // frames of one class may share a batch launch
+size_t pw_tc_operand_bytes(int na, int K, int ne_pad);   // bytes of tc_B
+size_t pw_tc_scratch_bytes(int grid);                    // bytes of u_scr
+int pw_tc_grid(const PWDev& d);
+int pw_tc_items(const PWDev& d);
+int pw_tc_batch_grid();
+void pw_tc_pick_split(PWDev& d);
+// window table of the columns wt_c0 .. wt_c0 + wt_nc - 1
+cudaError_t launch_pw_tc_window(const PWDev& d, float* tab, float* sum, cudaStream_t s);
+// the spectra's scale and B tiles; widest: the largest angle count of the launch that reads
+// them (0: the frame's own)
+cudaError_t launch_pw_tc_operand(const PWDev& d, int widest, cudaStream_t s);
+// stack: one image per angle
+cudaError_t launch_pw_tc(const PWDev& d, bool stack, float2* image, float* weights, cudaStream_t s);
+cudaError_t launch_pw_tc_batch(const PWBatchDev& B, int widest, int grid, cudaStream_t s);
 cudaError_t launch_pw_plain(const PWDev& d, float2* image, float* weights, cudaStream_t s);
 constexpr int M_MAXE = 256;   // elements supported by the das_pw.m-semantics kernel
 cudaError_t launch_pw_m(const PWDev& d, int compound, float2* image, float* weights, cudaStream_t s);

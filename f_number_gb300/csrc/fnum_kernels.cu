@@ -11,8 +11,10 @@
 //                        das_kernel_normalization (+cuda/gpu_bf_das_pw_rf.cu:965-1057)
 //   pw_event_kernel      the same recurrence with the segment boundaries resolved ahead
 //                        of the bin loop
-//   pw_tc_kernel         the same image from per-bin [voxels x elements] . [elements x
-//                        angles] products on the tensor cores (mma.sync, fp16 hi/lo)
+//   pw_mma_kernel, pw_mma_deriv_kernel
+//                        the same image from per-bin [voxels x elements] . [elements x
+//                        angles] products (mma.sync, fp16 hi/lo) for the differentiable
+//                        binding; the other images' products are fnum_pw_tc.cu's (tcgen05)
 //   sa_fused_kernel      the recurrence for synthetic-aperture data
 //                        (+cuda/gpu_bf_saft_rf.cu:1144-1201, saft_kernel_phase_shifts.cu)
 //   sa_event_kernel      the same for a boxcar receive window, boundaries resolved ahead
@@ -778,6 +780,13 @@ pw_event_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ w
 // ---------------------------------------------------------------------------
 // plane-wave kernel on the tensor cores
 // ---------------------------------------------------------------------------
+// plane-wave image and derivative with warp-level mma.sync
+// ---------------------------------------------------------------------------
+// The differentiable binding's forward pass and dL/dc.  Its loss and dL/dc are FP64 values
+// that callers compare between versions to 1e-9, which fixes the rounding of every step
+// below them, so this path keeps its arithmetic; every other image comes from the kernel of
+// fnum_pw_tc.cu (150 x 203 voxels, 96 elements, 5 angles: 2.1 ms here, 1.2 ms there).
+//
 // Per bin k the compounded image gains
 //   sum_a t_{v,a}^k G_k(v, a),   G_k(v, a) = sum_e R_k(v, e) X_k(e, a),
 //   R_k(v, e) = b_{v,e,k} r_{v,e}^k,
@@ -806,21 +815,6 @@ __device__ __forceinline__ void tc_split(float x0, float x1, unsigned& hi, unsig
   const __half2 l = __floats2half2_rn(x0 - f.x, x1 - f.y);
   hi = *reinterpret_cast<const unsigned*>(&h);
   lo = *reinterpret_cast<const unsigned*>(&l);
-}
-
-// the same split with the residual from sm_100's mixed-precision FMA: lo = x - hi
-// in one instruction per value (fp16 source, fp32 result; x - hi is exact, so the
-// halves are those of tc_split)
-__device__ __forceinline__ void tc_split_mx(float x0, float x1, unsigned& hi, unsigned& lo) {
-  asm("{\n\t.reg .b16 h0, h1, m;\n\t.reg .f32 l0, l1;\n\t"
-      "cvt.rn.f16x2.f32 %0, %3, %2;\n\t"
-      "mov.b32 {h0, h1}, %0;\n\t"
-      "mov.b16 m, 0xBC00;\n\t"
-      "fma.rn.f32.f16 l0, h0, m, %2;\n\t"
-      "fma.rn.f32.f16 l1, h1, m, %3;\n\t"
-      "cvt.rn.f16x2.f32 %1, l1, l0;\n\t}"
-      : "=&r"(hi), "=r"(lo)
-      : "f"(x0), "f"(x1));
 }
 
 // D += A B for one m16n8k16 tile (row-major A, column-major B, fp32 accumulators)
@@ -882,7 +876,7 @@ __global__ void __launch_bounds__(256) tc_prep_kernel(const PWDev d, int n_ap, i
   d.tc_B[i] = o;
 }
 
-// Shared memory of pw_tc_kernel's tile body.
+// Shared memory of pw_mma_kernel's tile body.
 struct TcShared {
   float4 apt[TC_WARPS][TC_TT][16];   // {segment index (int bits), 1/L_left, 1/L_right, 1/W} per bin, voxel
   int e_range[2];
@@ -923,12 +917,7 @@ struct TcDerivShared {
 // a second Horner chain beside each first one: going down the bins, Q <- (Q + P) t
 // before P <- P t + Y, and a chunk ending at bin kc_lo contributes t^kc_lo (kc_lo P + Q).
 // dimage receives Draw (scaled like the image).
-//
-// BATCH (the persistent batch kernel, whose descriptor lies in global memory) reads the
-// descriptor fields used at every bin (k_lb, tc_S) once per tile; the per-frame kernels
-// read their parameters' fields where they are used (constant-bank operands, no
-// registers held).
-template <int WIN, bool DERIV, bool BATCH = false, int NT = 3>
+template <int WIN, bool DERIV, int NT = 3>
 __device__ __forceinline__ void pw_tc_tile(const PWDev& d, int tile, int n_tiles_x, int n_tiles_z, TcShared& sh,
                                            const dfl* lb_s, const dfl* ub_s, int* ktop, float2* __restrict__ image,
                                            float* __restrict__ weights, unsigned long long& n_active,
@@ -950,8 +939,6 @@ __device__ __forceinline__ void pw_tc_tile(const PWDev& d, int tile, int n_tiles
   int4* seg_blk = d.seg + (size_t)blockIdx.x * NTHREADS * (size_t)d.seg_cap * PW_SEG_INT4;
   const float inv_par = (d.window_par > 0.0f) ? 1.0f / d.window_par : 0.0f;
   const float inv_sigma = 1.0f / tc_scale(*d.tc_max);
-  const int b_k_lb = d.k_lb, b_tc_S = d.tc_S;
-#define TC_D(field) (BATCH ? b_##field : d.field)
   const int tb = (d.tc_tb > 0 && d.tc_tb < TC_TB) ? d.tc_tb : TC_TB;   // bins per flush (a launch shape)
   constexpr int NA_P = 4 * NT;     // angles per pass
   constexpr int NB = 32 * NT;      // uint4 of B fragments per element group and bin
@@ -1025,7 +1012,7 @@ __device__ __forceinline__ void pw_tc_tile(const PWDev& d, int tile, int n_tiles
       for (int e0 = E_lo; e0 <= E_hi; e0 += TC_EP) {
         int kt = -1;
         for (int e = max(e0, 0); e < min(e0 + TC_EP, E_hi + 1); ++e) kt = max(kt, ktop[e]);
-        if (kt < TC_D(k_lb)) continue;
+        if (kt < d.k_lb) continue;
         if (tid == 0)
           n_exec += (unsigned long long)(kt - d.k_lb + 1) * TC_EP * min(NA_P, d.na - a0) * (TC_WARPS * 16);
         // the thread's (voxel, element) pairs: V, element e0 + 8s + 2q + i
@@ -1082,8 +1069,8 @@ __device__ __forceinline__ void pw_tc_tile(const PWDev& d, int tile, int n_tiles
         // the pairs' weights of the segment in effect, recomputed when a voxel enters a new segment
         float bw[2][TC_KS][2];
         int wid[2] = {-1, -1};
-        for (int kc_hi = kt; kc_hi >= TC_D(k_lb); kc_hi -= tb) {
-          const int kc_lo = max(TC_D(k_lb), kc_hi - (tb - 1));
+        for (int kc_hi = kt; kc_hi >= d.k_lb; kc_hi -= tb) {
+          const int kc_lo = max(d.k_lb, kc_hi - (tb - 1));
           // receive phasors re-anchored exactly at the chunk's first bin
 #pragma unroll
           for (int V = 0; V < 2; ++V) {
@@ -1162,7 +1149,7 @@ __device__ __forceinline__ void pw_tc_tile(const PWDev& d, int tile, int n_tiles
                   H[j][2 * V] = fmaf(hr, t.x, -hi * t.y);
                   H[j][2 * V + 1] = fmaf(hr, t.y, hi * t.x);
                 }
-              const uint4* Bk = Bpe + (size_t)(k - TC_D(k_lb)) * TC_D(tc_S) * NB;
+              const uint4* Bk = Bpe + (size_t)(k - d.k_lb) * d.tc_S * NB;
 #pragma unroll
               for (int s = 0; s < TC_KS; ++s) {
                 uint4 bf[NT];
@@ -1292,10 +1279,9 @@ __device__ __forceinline__ void pw_tc_tile(const PWDev& d, int tile, int n_tiles
     __syncthreads();
   }
 }
-#undef TC_D
 
 // the per-frame statistics of pw_tc_tile, added to the frame's counters
-__device__ __forceinline__ void pw_tc_flush_counts(const PWDev& d, unsigned long long& n_active,
+__device__ __forceinline__ void pw_mma_flush_counts(const PWDev& d, unsigned long long& n_active,
                                                    unsigned long long& n_empty, unsigned long long& n_exec) {
   atomicAdd(&d.counters[0], n_active * (unsigned long long)d.na);
   atomicAdd(&d.counters[1], n_empty * (unsigned long long)d.na);
@@ -1305,7 +1291,7 @@ __device__ __forceinline__ void pw_tc_flush_counts(const PWDev& d, unsigned long
 
 template <int WIN, int NT>
 __global__ void __launch_bounds__(NTHREADS, 4)
-pw_tc_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ weights, int n_tiles_x, int n_tiles_z) {
+pw_mma_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ weights, int n_tiles_x, int n_tiles_z) {
   __shared__ TcShared sh;
   __shared__ int s_tile;
   extern __shared__ __align__(16) unsigned char dyn[];  // lb[ne], ub[ne] (dfl), ktop[ne]
@@ -1329,73 +1315,16 @@ pw_tc_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ weig
     __syncthreads();
     const int tile = s_tile;
     if (tile >= n_tiles) break;
-    pw_tc_tile<WIN, false, false, NT>(d, tile, n_tiles_x, n_tiles_z, sh, lb_s, ub_s, ktop, image, weights, n_active,
+    pw_tc_tile<WIN, false, NT>(d, tile, n_tiles_x, n_tiles_z, sh, lb_s, ub_s, ktop, image, weights, n_active,
                                       n_empty, n_exec);
   }
-  pw_tc_flush_counts(d, n_active, n_empty, n_exec);
-}
-
-// One persistent launch over the tiles of many frames (a batch): each block draws
-// global tile numbers from the batch's counter, in frame order (the host orders the
-// frames largest first), finds the tile's frame, and runs pw_tc_tile on it.  The frames'
-// descriptors stay in device memory (read through the cache; the host has set their
-// segment scratch to the batch's), which measured faster than a copy in shared memory.
-template <int WIN, int NT>
-__global__ void __launch_bounds__(NTHREADS, 4) pw_tc_batch_kernel(const PWBatchDev B) {
-  __shared__ TcShared sh;
-  __shared__ int s_tile, s_frame;
-  extern __shared__ __align__(16) unsigned char dyn[];  // lb[max_ne], ub[max_ne] (dfl), ktop[max_ne]
-  dfl* lb_s = (dfl*)dyn;
-  dfl* ub_s = lb_s + B.max_ne;
-  int* ktop = (int*)(ub_s + B.max_ne);
-  const int tid = threadIdx.x;
-  unsigned long long n_active = 0, n_empty = 0, n_exec = 0;
-  int cur = -1;
-  for (;;) {
-    if (tid == 0) {
-      const int t = (int)atomicAdd(B.counter, 1ull);
-      int f = -1;
-      if (t < B.tile_start[B.n_frames]) {
-        int lo = 0, hi = B.n_frames - 1;   // the frame whose tile range holds t
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (B.tile_start[mid] <= t) lo = mid; else hi = mid - 1;
-        }
-        f = lo;
-        s_tile = t - B.tile_start[f];
-      }
-      s_frame = f;
-    }
-    __syncthreads();
-    const int f = s_frame;
-    if (f < 0) break;
-    const PWDev& d = B.frames[f];
-    if (f != cur) {
-      if (cur >= 0) pw_tc_flush_counts(B.frames[cur], n_active, n_empty, n_exec);
-      __syncthreads();   // every thread is done with the previous frame's element edges
-      for (int e = tid; e < d.ne; e += NTHREADS) {
-        lb_s[e] = d.el_lb[e];
-        ub_s[e] = d.el_ub[e];
-      }
-      cur = f;
-    }
-    for (int e = tid; e < B.max_ne; e += NTHREADS) ktop[e] = -1;
-    if (tid == 0) {
-      sh.e_range[0] = d.ne;
-      sh.e_range[1] = -1;
-    }
-    __syncthreads();
-    const int ntx = (d.nx + TC_TILE_X - 1) / TC_TILE_X, ntz = (d.nz + TILE_Z - 1) / TILE_Z;
-    pw_tc_tile<WIN, false, true, NT>(d, s_tile, ntx, ntz, sh, lb_s, ub_s, ktop, B.images[f], B.weights[f], n_active, n_empty,
-                           n_exec);
-  }
-  if (cur >= 0) pw_tc_flush_counts(B.frames[cur], n_active, n_empty, n_exec);
+  pw_mma_flush_counts(d, n_active, n_empty, n_exec);
 }
 
 // The image and its derivative with respect to the speed of sound (see pw_tc_tile).
 template <int WIN>
 __global__ void __launch_bounds__(NTHREADS, 3)
-pw_tc_deriv_kernel(const PWDev d, float2* __restrict__ image, float2* __restrict__ dimage, int n_tiles_x,
+pw_mma_deriv_kernel(const PWDev d, float2* __restrict__ image, float2* __restrict__ dimage, int n_tiles_x,
                    int n_tiles_z) {
   __shared__ TcShared sh;
   __shared__ int s_tile;
@@ -1424,7 +1353,7 @@ pw_tc_deriv_kernel(const PWDev d, float2* __restrict__ image, float2* __restrict
     pw_tc_tile<WIN, true>(d, tile, n_tiles_x, n_tiles_z, sh, lb_s, ub_s, ktop, image, nullptr, n_active, n_empty,
                           n_exec, &dsh, dimage);
   }
-  pw_tc_flush_counts(d, n_active, n_empty, n_exec);
+  pw_mma_flush_counts(d, n_active, n_empty, n_exec);
 }
 
 typedef void (*pw_kernel_t)(const PWDev, float2*, float*, int, int);
@@ -1454,26 +1383,13 @@ static pw_kernel_t pw_pick_event_win(int window_id) {
 //     1: EPT 1 x NA 11   2: EPT 2 x NA 4   3: EPT 2 x NA 2   4: EPT 4 x NA 1
 //   boundaries resolved inside the bin loop (pw_fused_kernel):
 //     5: EPT 1 x NA 11   6: EPT 2 x NA 4   7: EPT 2 x NA 2   8: EPT 4 x NA 1
-//   9: tensor cores (pw_tc_kernel), 16 elements x 12 angles per pass, or 16
-//      angles where that takes fewer passes (PWDev::tc_nt); needs the plan's
-//      fragment scratch (PWDev::tc_B)
+//   9: tensor cores (fnum_pw_tc.cu), up to 32 angles per pass; needs the plan's
+//      operand scratch (PWDev::tc_B)
 // Angles beyond NA run as further passes inside the launch.  PWDev::variant
 // 0 picks by the angle count; a plan's autotuner may set another.
-static pw_kernel_t pw_pick_tc_win(int window_id, int nt) {
-  const bool n4 = nt == 4;
-  switch (window_id) {
-    case 0: return n4 ? pw_tc_kernel<0, 4> : pw_tc_kernel<0, 3>;
-    case 1: return n4 ? pw_tc_kernel<1, 4> : pw_tc_kernel<1, 3>;
-    case 2: return n4 ? pw_tc_kernel<2, 4> : pw_tc_kernel<2, 3>;
-    default: return n4 ? pw_tc_kernel<4, 4> : pw_tc_kernel<4, 3>;
-  }
-}
-// n-tiles per angle pass of frame d's tensor-core kernel (tc_ntiles_for, set at plan creation)
-static int pw_tc_nt(const PWDev& d) { return d.tc_nt == 4 ? 4 : 3; }
 static pw_kernel_t pw_variant_kernel(int v, const PWDev& d) {
   const int window_id = d.window_id;
   switch (v) {
-    case TC_VARIANT: return pw_pick_tc_win(window_id, pw_tc_nt(d));
     case 1: return pw_pick_event_win<1, 11>(window_id);
     case 2: return pw_pick_event_win<2, 4>(window_id);
     case 3: return pw_pick_event_win<2, 2>(window_id);
@@ -1484,30 +1400,66 @@ static pw_kernel_t pw_variant_kernel(int v, const PWDev& d) {
     default: return pw_pick_win<4, 1>(window_id);
   }
 }
-// default pass shape by angle count; with the fragment scratch in place the
-// tensor-core variant from 3 angles on (measured at 128 elements, 256 x 256)
+static int pw_fp32_variant(const PWDev& d) { return d.na >= 11 ? 1 : (d.na >= 4 ? 2 : (d.na >= 2 ? 3 : 4)); }
+// Default pass shape.  With the operand scratch in place the tensor cores take three angles
+// or more (11 angles of 128 elements on 512 x 512: 16.2 ms, the FP32 kernel 57 ms).  They run
+// one or two angles in the time of eight, the FP32 kernels in proportion, but on few tiles
+// those are bound by one tile's serial chain, which grows with the elements.  Measured,
+// FP32 | tensor cores, 2-7 MHz band:
+//   one angle, 128 elements: 24^2 5819 | 363 us, 256^2 4555 | 4175, 400^2 9141 | 9969
+//              64 elements:  24^2 2353 | 219,    128^2 1904 | 695,  400^2 3887 | 5061
+//   two angles, 128:         128^2 4700 | 1285,  400^2 13018 | 9973
+//               64:          128^2 2407 | 701,   400^2 5742 | 5064
+//               48:          128^2 1735 | 564,   400^2 4094 | 4097
+// so the crossing lies near 6 tiles (of 128 voxels) an element for one angle, and for two at
+// 64 elements.  Probes of up to 32 elements keep the FP32 kernel, which a batch runs beside
+// its persistent launches (24^2: 1229 | 151 us, 400^2: 1802 | 3131).
 static int pw_default_variant(const PWDev& d) {
-  if (d.tc_B && d.na >= 3) return TC_VARIANT;
-  if (d.na >= 11) return 1;
-  if (d.na >= 4) return 2;
-  if (d.na >= 2) return 3;
-  return 4;
+  if (d.tc_B) {
+    if (d.na >= 3) return TC_VARIANT;
+    const long long tiles = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
+    if (d.ne > 32 && ((d.na == 2 && d.ne >= 64) || tiles <= 6ll * d.na * d.ne)) return TC_VARIANT;
+  }
+  return pw_fp32_variant(d);
 }
 static pw_kernel_t pw_pick(const PWDev& d) {
   return pw_variant_kernel(d.variant > 0 ? d.variant : pw_default_variant(d), d);
 }
 int pw_variant_count() { return 9; }
+int pw_mma_variant_of(const PWDev& d) {
+  return d.variant > 0 ? d.variant : (d.tc_B && d.na >= 3 ? TC_VARIANT : pw_fp32_variant(d));
+}
 int pw_variant_of(const PWDev& d) { return d.variant > 0 ? d.variant : pw_default_variant(d); }
 
-static int pw_tiles_x(const PWDev& d) {
-  const int tw = pw_variant_of(d) == TC_VARIANT ? TC_TILE_X : TILE_X;
-  return (d.nx + tw - 1) / tw;
+static int pw_tiles_x(const PWDev& d) { return (d.nx + TILE_X - 1) / TILE_X; }
+
+// n-tiles per angle pass (tc_ntiles_for, set at plan creation)
+static int pw_mma_nt(const PWDev& d) { return d.tc_nt == 4 ? 4 : 3; }
+
+typedef void (*pw_mma_t)(const PWDev, float2*, float*, int, int);
+static pw_mma_t pw_mma_pick(const PWDev& d) {
+  const bool n4 = pw_mma_nt(d) == 4;
+  switch (d.window_id) {
+    case 0: return n4 ? pw_mma_kernel<0, 4> : pw_mma_kernel<0, 3>;
+    case 1: return n4 ? pw_mma_kernel<1, 4> : pw_mma_kernel<1, 3>;
+    case 2: return n4 ? pw_mma_kernel<2, 4> : pw_mma_kernel<2, 3>;
+    default: return n4 ? pw_mma_kernel<4, 4> : pw_mma_kernel<4, 3>;
+  }
+}
+typedef void (*pw_mma_deriv_t)(const PWDev, float2*, float2*, int, int);
+static pw_mma_deriv_t pw_mma_deriv_pick(int window_id) {
+  switch (window_id) {
+    case 0: return pw_mma_deriv_kernel<0>;
+    case 1: return pw_mma_deriv_kernel<1>;
+    case 2: return pw_mma_deriv_kernel<2>;
+    default: return pw_mma_deriv_kernel<4>;
+  }
 }
 
-// The tensor-core tile kernels' static shared memory and their element tables (20
-// bytes per element, dynamic) exceed the 48 KB a block may use without opting in:
-// each of them is allowed the device's maximum once per device.
-static cudaError_t pw_tc_smem_optin() {
+// Static shared memory and the element tables (20 bytes per element, dynamic) exceed the
+// 48 KB a block may use without opting in: each kernel is allowed the device's maximum once
+// per device.
+static cudaError_t pw_mma_smem_optin() {
   static std::mutex mu;
   static bool done[64] = {};
   int dev = 0;
@@ -1518,16 +1470,12 @@ static cudaError_t pw_tc_smem_optin() {
   int optin = 0;
   if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
   const void* fns[] = {
-      (const void*)pw_tc_kernel<0, 3>,       (const void*)pw_tc_kernel<1, 3>,
-      (const void*)pw_tc_kernel<2, 3>,       (const void*)pw_tc_kernel<4, 3>,
-      (const void*)pw_tc_kernel<0, 4>,       (const void*)pw_tc_kernel<1, 4>,
-      (const void*)pw_tc_kernel<2, 4>,       (const void*)pw_tc_kernel<4, 4>,
-      (const void*)pw_tc_batch_kernel<0, 3>, (const void*)pw_tc_batch_kernel<1, 3>,
-      (const void*)pw_tc_batch_kernel<2, 3>, (const void*)pw_tc_batch_kernel<4, 3>,
-      (const void*)pw_tc_batch_kernel<0, 4>, (const void*)pw_tc_batch_kernel<1, 4>,
-      (const void*)pw_tc_batch_kernel<2, 4>, (const void*)pw_tc_batch_kernel<4, 4>,
-      (const void*)pw_tc_deriv_kernel<0>,    (const void*)pw_tc_deriv_kernel<1>,
-      (const void*)pw_tc_deriv_kernel<2>,    (const void*)pw_tc_deriv_kernel<4>};
+      (const void*)pw_mma_kernel<0, 3>,      (const void*)pw_mma_kernel<1, 3>,
+      (const void*)pw_mma_kernel<2, 3>,      (const void*)pw_mma_kernel<4, 3>,
+      (const void*)pw_mma_kernel<0, 4>,      (const void*)pw_mma_kernel<1, 4>,
+      (const void*)pw_mma_kernel<2, 4>,      (const void*)pw_mma_kernel<4, 4>,
+      (const void*)pw_mma_deriv_kernel<0>,   (const void*)pw_mma_deriv_kernel<1>,
+      (const void*)pw_mma_deriv_kernel<2>,   (const void*)pw_mma_deriv_kernel<4>};
   for (const void* f : fns) {
     cudaFuncAttributes a;
     if ((e = cudaFuncGetAttributes(&a, f)) != cudaSuccess) return e;
@@ -1539,10 +1487,61 @@ static cudaError_t pw_tc_smem_optin() {
   return cudaSuccess;
 }
 
+// a grid with all blocks resident
+static int pw_mma_grid(const PWDev& d, const void* fn, size_t smem) {
+  int dev = 0, nsm = 0, bps = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, NTHREADS, smem);
+  if (bps < 1) bps = 1;
+  return min(((d.nx + TC_TILE_X - 1) / TC_TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z), nsm * bps);
+}
+static size_t pw_mma_smem(const PWDev& d) { return (size_t)d.ne * (sizeof(int) + 2 * sizeof(dfl)); }
+
+static cudaError_t launch_pw_mma_prep(const PWDev& d, cudaStream_t s, int nt) {
+  if (!d.tc_B || !d.tc_max) return cudaErrorInvalidValue;
+  // spectra -> fp16 B fragments, scaled by a power of two set by their largest component
+  cudaError_t e = cudaMemsetAsync(d.tc_max, 0, sizeof(unsigned), s);
+  if (e != cudaSuccess) return e;
+  tc_absmax_kernel<<<304, 256, 0, s>>>(d, d.tc_max);
+  const int n_ap = (d.na + 4 * nt - 1) / (4 * nt);
+  const size_t n = (size_t)n_ap * d.K * d.tc_S * nt * 32;
+  tc_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, n_ap, nt);
+  return cudaGetLastError();
+}
+
+// max_grid: blocks that the plan's segment scratch holds
+cudaError_t launch_pw_mma(const PWDev& d, int max_grid, float2* image, cudaStream_t s) {
+  cudaError_t e = pw_mma_smem_optin();
+  if (e == cudaSuccess) e = launch_pw_mma_prep(d, s, pw_mma_nt(d));
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.counters + 3, 0, sizeof(unsigned long long), s);
+  if (e != cudaSuccess) return e;
+  const size_t smem = pw_mma_smem(d);
+  const pw_mma_t fn = pw_mma_pick(d);
+  const int ntx = (d.nx + TC_TILE_X - 1) / TC_TILE_X, ntz = (d.nz + TILE_Z - 1) / TILE_Z;
+  fn<<<min(pw_mma_grid(d, (const void*)fn, smem), max_grid), NTHREADS, smem, s>>>(d, image, nullptr, ntx, ntz);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pw_mma_deriv(const PWDev& d, int max_grid, float2* image, float2* dimage, cudaStream_t s) {
+  cudaError_t e = pw_mma_smem_optin();
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.counters, 0, 5 * sizeof(unsigned long long), s);
+  if (e == cudaSuccess) e = launch_pw_mma_prep(d, s, 3);   // passes of 12 angles
+  if (e != cudaSuccess) return e;
+  const size_t smem = sizeof(TcDerivShared) + pw_mma_smem(d);
+  const pw_mma_deriv_t fn = pw_mma_deriv_pick(d.window_id);
+  const int ntx = (d.nx + TC_TILE_X - 1) / TC_TILE_X, ntz = (d.nz + TILE_Z - 1) / TILE_Z;
+  fn<<<min(pw_mma_grid(d, (const void*)fn, smem), max_grid), NTHREADS, smem, s>>>(d, image, dimage, ntx, ntz);
+  return cudaGetLastError();
+}
+
 int pw_fused_grid(const PWDev& d, int* blocks_per_sm) {
+  if (pw_variant_of(d) == TC_VARIANT) {
+    if (blocks_per_sm) *blocks_per_sm = 1;
+    return pw_tc_grid(d);
+  }
   pw_kernel_t fn = pw_pick(d);
   int dev = 0, nsm = 0, bps = 0;
-  (void)pw_tc_smem_optin();
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, NTHREADS, (size_t)d.ne * (sizeof(int) + 2 * sizeof(dfl)));
@@ -1555,102 +1554,28 @@ int pw_fused_grid(const PWDev& d, int* blocks_per_sm) {
 
 int pw_fused_max_grid(const PWDev& d) {
   int g = 0;
-  for (int v = 1; v <= pw_variant_count(); ++v) {
+  for (int v = 1; v < TC_VARIANT; ++v) {
     PWDev t = d;
     t.variant = v;
     t.blocks_per_sm = 0;
     g = max(g, pw_fused_grid(t, nullptr));
   }
+  if (pw_mma_smem_optin() == cudaSuccess)
+    g = max(g, pw_mma_grid(d, (const void*)pw_mma_pick(d), pw_mma_smem(d)));
   return g;
 }
 
 cudaError_t launch_pw_fused(const PWDev& d, int grid, float2* image, float* weights, cudaStream_t s) {
+  if (pw_variant_of(d) == TC_VARIANT) return launch_pw_tc(d, false, image, weights, s);
   const int ntx = pw_tiles_x(d), ntz = (d.nz + TILE_Z - 1) / TILE_Z;
   const size_t smem = (size_t)d.ne * (sizeof(int) + 2 * sizeof(dfl));
   // each launch draws tiles from a fresh counter
-  cudaError_t e = pw_tc_smem_optin();
-  if (e == cudaSuccess) e = cudaMemsetAsync(d.counters + 3, 0, sizeof(unsigned long long), s);
+  cudaError_t e = cudaMemsetAsync(d.counters + 3, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  if (pw_variant_of(d) == TC_VARIANT && (e = launch_pw_tc_prep(d, s)) != cudaSuccess) return e;
   pw_pick(d)<<<grid, NTHREADS, smem, s>>>(d, image, weights, ntx, ntz);
   return cudaGetLastError();
 }
 
-cudaError_t launch_pw_tc_prep(const PWDev& d, cudaStream_t s, int nt) {
-  if (!d.tc_B || !d.tc_max) return cudaErrorInvalidValue;
-  if (nt != 3 && nt != 4) nt = pw_tc_nt(d);
-  // spectra -> fp16 B fragments, scaled by a power of two set by their largest component
-  cudaError_t e = cudaMemsetAsync(d.tc_max, 0, sizeof(unsigned), s);
-  if (e != cudaSuccess) return e;
-  tc_absmax_kernel<<<304, 256, 0, s>>>(d, d.tc_max);
-  const int n_ap = (d.na + 4 * nt - 1) / (4 * nt);
-  const size_t n = (size_t)n_ap * d.K * d.tc_S * nt * 32;
-  tc_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, n_ap, nt);
-  return cudaGetLastError();
-}
-
-typedef void (*pw_tc_deriv_t)(const PWDev, float2*, float2*, int, int);
-static pw_tc_deriv_t pw_tc_deriv_pick(int window_id) {
-  switch (window_id) {
-    case 0: return pw_tc_deriv_kernel<0>;
-    case 1: return pw_tc_deriv_kernel<1>;
-    case 2: return pw_tc_deriv_kernel<2>;
-    default: return pw_tc_deriv_kernel<4>;
-  }
-}
-
-cudaError_t launch_pw_tc_deriv(const PWDev& d, float2* image, float2* dimage, cudaStream_t s) {
-  if (!d.tc_B || !d.tc_max) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(d.counters, 0, 5 * sizeof(unsigned long long), s);
-  if (e == cudaSuccess) e = launch_pw_tc_prep(d, s, 3);   // the derivative kernel runs passes of 12 angles
-  if (e != cudaSuccess) return e;
-  const size_t smem = sizeof(TcDerivShared) + (size_t)d.ne * (sizeof(int) + 2 * sizeof(dfl));
-  if ((e = pw_tc_smem_optin()) != cudaSuccess) return e;
-  int dev = 0, nsm = 0, bps = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, pw_tc_deriv_pick(d.window_id), NTHREADS, smem);
-  if (bps < 1) bps = 1;
-  const int ntx = (d.nx + TC_TILE_X - 1) / TC_TILE_X, ntz = (d.nz + TILE_Z - 1) / TILE_Z;
-  // the plan's segment scratch holds pw_fused_max_grid blocks: at least this many
-  const int grid = min(min(ntx * ntz, nsm * bps), pw_fused_max_grid(d));
-  pw_tc_deriv_pick(d.window_id)<<<grid, NTHREADS, smem, s>>>(d, image, dimage, ntx, ntz);
-  return cudaGetLastError();
-}
-
-int pw_tc_tiles(const PWDev& d) { return ((d.nx + TC_TILE_X - 1) / TC_TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z); }
-
-typedef void (*pw_tc_batch_t)(const PWBatchDev);
-static pw_tc_batch_t pw_tc_batch_pick(int window_id, int nt) {
-  const bool n4 = nt == 4;
-  switch (window_id) {
-    case 0: return n4 ? pw_tc_batch_kernel<0, 4> : pw_tc_batch_kernel<0, 3>;
-    case 1: return n4 ? pw_tc_batch_kernel<1, 4> : pw_tc_batch_kernel<1, 3>;
-    case 2: return n4 ? pw_tc_batch_kernel<2, 4> : pw_tc_batch_kernel<2, 3>;
-    default: return n4 ? pw_tc_batch_kernel<4, 4> : pw_tc_batch_kernel<4, 3>;
-  }
-}
-
-int pw_tc_batch_grid(int max_ne, int window_id, int nt, int* blocks_per_sm) {
-  int dev = 0, nsm = 0, bps = 0;
-  (void)pw_tc_smem_optin();
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, pw_tc_batch_pick(window_id, nt), NTHREADS,
-                                                (size_t)max_ne * (sizeof(int) + 2 * sizeof(dfl)));
-  if (bps < 1) bps = 1;
-  if (blocks_per_sm) *blocks_per_sm = bps;
-  return nsm * bps;
-}
-
-cudaError_t launch_pw_tc_batch(const PWBatchDev& B, int window_id, int nt, int grid, cudaStream_t s) {
-  cudaError_t e = pw_tc_smem_optin();
-  if (e == cudaSuccess) e = cudaMemsetAsync(B.counter, 0, sizeof(unsigned long long), s);
-  if (e != cudaSuccess) return e;
-  const size_t smem = (size_t)B.max_ne * (sizeof(int) + 2 * sizeof(dfl));
-  pw_tc_batch_pick(window_id, nt)<<<grid, NTHREADS, smem, s>>>(B);
-  return cudaGetLastError();
-}
 // ---------------------------------------------------------------------------
 // plain per-voxel plane-wave kernel (reference arithmetic per term)
 // ---------------------------------------------------------------------------

@@ -1,6 +1,6 @@
 // Inline-PTX building blocks of the Blackwell tensor-core kernels (the band DFT,
-// fnum_dft_tc.cu, and the synthetic-aperture beamformer, fnum_sa_tc.cu):
-// mbarriers with bounded waits, TMA tile loads, shared-memory matrix
+// fnum_dft_tc.cu, and the plane-wave and synthetic-aperture beamformers, fnum_pw_tc.cu and
+// fnum_sa_tc.cu): mbarriers with bounded waits, TMA tile and bulk loads, shared-memory matrix
 // descriptors, tcgen05.mma / commit and tensor-memory loads and stores.
 #pragma once
 #include <cuda.h>
@@ -107,6 +107,42 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t da, uint64_t d
       "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
 }
 
+// D (tensor memory) = A B (+ D if accumulate), A from tensor memory (row = lane, two
+// consecutive K values per 32-bit column), B from shared memory
+__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(
+          tmem_d),
+      "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate));
+}
+
+// an arrival of the lanes whose `on` is not 0 (a warp may run it converged with one such lane)
+__device__ __forceinline__ void mbar_arrive_if(uint32_t on, uint32_t bar) {
+  asm volatile(
+      "{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n@q mbarrier.arrive.shared::cta.b64 _, [%0];\n}\n" ::"r"(bar), "r"(on)
+      : "memory");
+}
+
+// shared-memory matrix descriptor without swizzle: core matrices of 8 rows x 16 bytes (128
+// contiguous bytes); lbo bytes between core matrices along K, sbo bytes between groups of 8 rows
+__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
+         ((uint64_t)1 << 46);
+}
+
+// its upper half (the lower: address and lbo)
+__host__ __device__ constexpr uint64_t smem_desc_plain_hi(uint32_t sbo) {
+  return ((uint64_t)(sbo >> 4) << 32) | ((uint64_t)1 << 46);
+}
+
+// contiguous global -> shared copy (16-byte aligned, a multiple of 16 bytes), counted by the mbarrier
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
 // the mbarrier receives one arrival once every tcgen05.mma issued so far by this thread is complete
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -143,6 +179,14 @@ __device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, float (&v)[8]) {
                : "r"(taddr));
 }
 
+// 4 consecutive columns of the warp's 32 lanes (no wait)
+__device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, float (&v)[4]) {
+  uint32_t* u = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3])
+               : "r"(taddr));
+}
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
@@ -153,6 +197,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
       "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]),
       "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
       : "memory");
+}
+
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&u)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+               "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7])
+               : "memory");
 }
 
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }

@@ -612,6 +612,13 @@ def _pw_set_spectra(self, spectra, stream=None):
     _lib.check(_lib.lib().fnum_plan_set_spectra(self._ptr, spectra.data_ptr(), self._stream_ptr(stream)))
 
 
+def _pw_forward(self, out, stream=None):
+    """The image of the plan's current spectra as the differentiable binding's forward
+    pass (fnum_pw_forward), into `out` (complex64 CUDA tensor [1, N_x, N_z])."""
+    _lib.check(_lib.lib().fnum_pw_forward(self._ptr, out.data_ptr(), self._stream_ptr(stream)))
+    return out
+
+
 def _pw_adjoint(self, cotangent, dc=True, stream=None):
     """Adjoint of the compounded beamformer (fnum_pw_adjoint): for G = dL/dI*
     (complex64 CUDA tensor [N_x, N_z]) at the plan's current spectra and sound
@@ -629,6 +636,7 @@ def _pw_adjoint(self, cotangent, dc=True, stream=None):
 PWPlan.set_sound_speed = _pw_set_sound_speed
 PWPlan.sharpness_grad = _pw_sharpness_grad
 PWPlan.set_spectra = _pw_set_spectra
+PWPlan.forward = _pw_forward
 PWPlan.adjoint = _pw_adjoint
 
 

@@ -275,10 +275,9 @@ int fnum_das_pw_noalloc(const fnum_pw_desc* desc, const double* steering_angles,
    variant of a plane-wave plan on it (1: 1 element x 11 angles per pass,
    2: 2 x 4, 3: 2 x 2, 4: 4 x 1, with the segment boundaries resolved ahead of
    the bin loop; 5..8: the same shapes resolving them inside the bin loop;
-   9: tensor cores, 16 elements x 12 angles per pass -- 16 angles where that
-   takes fewer passes -- the default from 3 angles on) at full occupancy, and
-   keeps the fastest
-   for the plan's later executes.  It allocates a temporary image and runs on
+   9: tensor cores, up to 32 angles per pass, the default from 3 angles on and for
+   one or two angles of more than 32 elements unless the grid is large) at full
+   occupancy, and keeps the fastest for the plan's later executes.  It allocates a temporary image and runs on
    a private stream (not capturable).  variant / ms (the chosen variant's
    beamform time) may be NULL.  A synthetic-aperture plan times its two
    variants (1: the per-pair recurrence kernels, 2: the tensor-core kernel, which
@@ -286,7 +285,7 @@ int fnum_das_pw_noalloc(const fnum_pw_desc* desc, const double* steering_angles,
    default when available); a FNUM_FLAG_PLAIN_KERNEL plan returns variant 0. */
 int fnum_plan_autotune(fnum_plan* plan, const void* d_rf, int rf_is_double, int* variant, float* ms);
 /* fnum_plan_set_kernel_variant: pins the fused-kernel variant of a plane-wave
-   plan (0 = by the angle count, 1..9 as above), e.g. one an earlier
+   plan (0 = by angles, elements and grid, 1..9 as above), e.g. one an earlier
    fnum_plan_autotune chose.  Every variant gives the same images up to the
    rounding of the per-pass sums.  A synthetic-aperture plan accepts 0 (default),
    1 and 2 (when available); a plan with FNUM_FLAG_M_SEMANTICS or
@@ -312,9 +311,9 @@ int fnum_plan_set_shape(fnum_plan* plan, int blocks_per_sm, int bin_chunk);
    frame's completion time in ms from the batch's start (n values, in the
    order of `plans`). */
 /* Compounded frames whose plans use the tensor-core kernel (variant 9) are not
-   launched per frame: their band DFTs and spectra fragments run on the branches,
-   then ONE persistent launch per window type and pass width (12 or 16 angles
-   per pass) beamforms all of them -- each block
+   launched per frame: their band DFTs and spectra operands run on the branches,
+   then ONE persistent launch per class of angle counts (up to 16, more)
+   beamforms all of them -- each block
    draws tiles of all those frames from one counter, largest frames first, with
    each frame's descriptor read from device memory -- so no SM idles between
    frames.  The other frames keep a launch per frame on the other branches.
@@ -366,6 +365,13 @@ int fnum_pw_sharpness_grad(fnum_plan* plan, const void* d_rf, int rf_is_double, 
    for the beamformer A.  Allocates the plan's gradient buffers on first use;
    synchronises `stream`. */
 int fnum_pw_adjoint(fnum_plan* plan, const void* d_cotangent, void* d_grad_spectra, double* dloss_dc, void* stream);
+/* The image of a compounded plane-wave plan's current spectra (device float2
+   [n_x][n_z]) as the forward pass of a differentiable binding: the rounding of this
+   image, and with it that of FP64 losses formed from it and of fnum_pw_adjoint's
+   dL/dc, is kept between versions, so from three angles on it comes from an
+   mma.sync kernel where fnum_plan_execute_beamform runs variant 9 (equal up to
+   rounding).  No counterpart in the reference. */
+int fnum_pw_forward(fnum_plan* plan, void* d_image, void* stream);
 /* loads band spectra (device float2, the layout of fnum_plan_spectra) into the
    plan, e.g. to beamform spectra a caller produced (fnum_plan_execute_beamform)
    or to take fnum_pw_adjoint at them.  No counterpart in the reference. */
