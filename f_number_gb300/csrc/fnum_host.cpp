@@ -673,6 +673,37 @@ int setup_pw_tc(fnum_plan* P, int na, int n_img) {
   return FNUM_OK;
 }
 
+// The same of a synthetic-aperture plan (equal windows share a table); bytes receives its size.
+int setup_sa_tc(fnum_plan* P, size_t* bytes) {
+  fnum::SADev& D = P->sa;
+  const int ne = D.ne;
+  const bool one = D.wtx_id == D.wrx_id && D.wtx_par == D.wrx_par;
+  D.ne_pad = (ne + 15) / 16 * 16;
+  const size_t col = (size_t)(ne + 1) * D.ne_pad;
+  const size_t fit = std::max<size_t>((((size_t)256 << 20) / (col * sizeof(float))) / 4 * 4, 4);
+  D.wt_c0 = 0;
+  D.wt_nc = (int)std::min<size_t>(fit, D.nx);
+  fnum::sa_tc_pick_split(D);
+  const size_t tiles = (size_t)((D.nx + fnum::TILE_X - 1) / fnum::TILE_X) * ((D.nz + fnum::TILE_Z - 1) / fnum::TILE_Z);
+  const size_t n_tab = col * D.wt_nc * sizeof(float), n_sum = (size_t)(ne + 1) * D.wt_nc * sizeof(float);
+  const size_t sizes[] = {n_tab, n_sum, one ? 0 : n_tab, one ? 0 : n_sum, fnum::sa_tc_scratch_bytes(D),
+                          D.split > 1 ? (size_t)D.split * D.nx * D.nz * sizeof(float2) : 0, tiles * sizeof(unsigned)};
+  size_t off[8] = {0};
+  for (int i = 0; i < 7; ++i) off[i + 1] = off[i] + (sizes[i] + 255) / 256 * 256;
+  unsigned char* m = nullptr;
+  if (const int s = P->alloc(&m, off[7])) return s;
+  for (int i = 0; i < 2; ++i) {
+    D.w_tab[i] = (float*)(m + off[one ? 0 : 2 * i]);
+    D.w_sum[i] = (float*)(m + off[one ? 1 : 2 * i + 1]);
+  }
+  D.u_scr = (float4*)(m + off[4]);
+  D.part = (float2*)(m + off[5]);
+  D.tile_cnt = (unsigned*)(m + off[6]);
+  *bytes = off[7];
+  if (D.wt_nc == D.nx) FNUM_CUDA(fnum::launch_sa_tc_window(D, 0));
+  return FNUM_OK;
+}
+
 int make_pw_plan(const fnum_pw_desc* d, const double* angles, int na, int flags, fnum_plan** out) {
   int s = check_pw(d, angles, na);
   if (s) return s;
@@ -946,9 +977,11 @@ int make_sa_plan(const fnum_sa_desc* d, int flags, fnum_plan** out) {
     }
     const size_t nb = fnum::sa_tc_bytes(ne, bk.K);
     if ((s = P->alloc(&planes, nb / 2)) || (s = P->alloc(&mb, 1)) || (s = P->upload(&rot, rv))) goto fail;
+    size_t n_more = 0;
+    if ((s = setup_sa_tc(P, &n_more))) goto fail;
     if (fnum::sa_tc_setup(P->satc, D, planes, mb, rot) == cudaSuccess) {
       P->sa_tc_ok = true;
-      P->info.scratch_bytes += (long long)nb;
+      P->info.scratch_bytes += (long long)(nb + n_more);
     } else {
       (void)cudaGetLastError();
     }
@@ -1002,8 +1035,7 @@ int plan_beamform(fnum_plan* P, void* image, float* w, float* w2, cudaStream_t s
     cudaError_t e;
     if (plain) e = fnum::launch_sa_plain(P->sa, (float2*)image, w, w2, st);
     else if (sa_variant_of(P) == 2)
-      e = fnum::launch_sa_tc(P->sa, P->satc, std::min(fnum::sa_tc_grid(P->sa), P->max_grid), (float2*)image, w, w2,
-                             st);
+      e = fnum::launch_sa_tc(P->sa, P->satc, (float2*)image, w, w2, st);
     else e = fnum::launch_sa_fused(P->sa, P->grid, (float2*)image, w, w2, st);
     return cuda_status(e);
   }

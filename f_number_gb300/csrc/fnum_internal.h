@@ -138,6 +138,15 @@ struct SADev {
   const float* px_f; const float* pz_f; const float* ctr_f; const float* lb_f; const float* ub_f;
   const float* Ftx_f; const float* Frx_f;
   float M_f, pitch_f, coef_f, add_f;
+  // tensor-core kernel (fnum_sa_tc.cu): as PWDev's, window tables of transmit and receive (equal
+  // pointers for equal windows)
+  const float* w_tab[2];
+  const float* w_sum[2];
+  int ne_pad, wt_c0, wt_nc;
+  float4* u_scr;
+  int split, split_bins;
+  float2* part;
+  unsigned* tile_cnt;
 };
 
 // One persistent launch of the tensor-core beamformer over the tiles of many
@@ -180,22 +189,22 @@ cudaError_t dft_tc_setup(DftTc& d, int nsig, int nt, int N, int k_lb, int K, con
 cudaError_t dft_tc_run(const DftTc& d, const void* rf, int is_double, float2* X, int lo_n, long long s_hi,
                        long long s_lo, long long s_k, unsigned long long* err, cudaStream_t s);
 
-// Synthetic-aperture beamformer on the tensor cores (fnum_sa_tc.cu): the spectra as
-// fp16 hi/lo planes [bin][2 nep][2 nep] in real form, their TMA maps, the scale word
-// and the time-offset phasors e^{2 pi i k t0 / N} of the band.
+// Synthetic-aperture beamformer on the tensor cores (fnum_sa_tc.cu): the spectra as fp16
+// hi/lo tiles in real form, the scale word and the time-offset phasors e^{2 pi i k t0 / N} of
+// the band.
 struct SaTc {
-  CUtensorMap tm[2];   // hi, lo (64-byte aligned)
   void* planes;
   unsigned* maxbits;
   const float2* rot;
-  int nep;             // elements rounded up to a multiple of 4
 };
 bool sa_tc_supported(const SADev& d);          // up to 128 elements, accumulating normalisations
-size_t sa_tc_bytes(int ne, int K);             // bytes of the planes
+size_t sa_tc_bytes(int ne, int K);             // bytes of the tiles
+size_t sa_tc_scratch_bytes(const SADev& d);    // bytes of u_scr
+void sa_tc_pick_split(SADev& d);
+cudaError_t launch_sa_tc_window(const SADev& d, cudaStream_t s);
 cudaError_t sa_tc_setup(SaTc& t, const SADev& d, void* planes, unsigned* maxbits, const float2* rot);
-int sa_tc_grid(const SADev& d);                // one block per SM (at most one per tile)
-cudaError_t launch_sa_tc(const SADev& d, const SaTc& t, int grid, float2* image, float* wtx, float* wrx,
-                         cudaStream_t s);
+int sa_tc_grid(const SADev& d);                // one block per SM (at most one per item)
+cudaError_t launch_sa_tc(const SADev& d, const SaTc& t, float2* image, float* wtx, float* wrx, cudaStream_t s);
 
 // --- launchers (fnum_kernels.cu) -------------------------------------------
 cudaError_t launch_twiddles(float2* tw, int N, cudaStream_t s);

@@ -1,4 +1,4 @@
-// The synthetic-aperture beamformer on the Blackwell tensor cores (tcgen05 + TMA).
+// The synthetic-aperture beamformer on the Blackwell tensor cores (tcgen05).
 //
 // Replaces the reference's per-bin, per-transmit phase matrices and cublasCgemm
 // calls (+cuda/gpu_bf_saft_rf.cu:1144-1201, +cuda/saft_kernel_phase_shifts.cu:8-199).
@@ -10,46 +10,53 @@
 // spectra), n_k = 1 / (W_tx W_rx) of the normalisations that are on, and
 // u_e(v) = |v - c_e| f_s / (N c) the one-way delay in cycles per bin.
 //
-// Y is a GEMM per bin: for a tile of 128 voxels (4 columns x 32 rows),
-//     D[v][2t + p] = sum_{r, q} A[v][2r + q] B[2t + p][2r + q]
+// Y is a GEMM per bin: for a tile of 128 voxels (4 columns x 32 rows, a voxel per TMEM lane)
+//     D[v][n(t, p)] = sum_{r, q} A[v][2r + q] B[n(t, p)][2r + q]
 // with A = (Re b_r, Im b_r) and B the real form of X'_k,
-//     B[2t][2r] = Re X', B[2t][2r+1] = -Im X', B[2t+1][2r] = Im X', B[2t+1][2r+1] = Re X',
-// so that D[v][2t] + i D[v][2t+1] = Y_t.  Both operands are split into fp16 hi +
-// lo parts (the spectra scaled by a power of two into fp16 range) and the products
-// hi.lo + lo.hi + hi.hi are accumulated in FP32 in tensor memory; the CUDA cores
-// only form the phasors and the dot products with a (O(elements) work per voxel
-// and bin, where the recurrence kernels do O(elements^2)).
+//     B[(t, 0)][(r, .)] = Re X', -Im X',   B[(t, 1)][(r, .)] = Im X', Re X',
+// so that D[v][(t, 0)] + i D[v][(t, 1)] = Y_t.  Both operands are split into fp16 hi + lo parts
+// (the spectra scaled by a power of two into fp16 range) and the products hi.lo + lo.hi + hi.hi
+// are accumulated in FP32 in tensor memory; the CUDA cores only form the phasors and the dot
+// products with a (O(elements) work per voxel and bin, where the recurrence kernels do
+// O(elements^2)).
 //
-// Kernel (persistent, one CTA per SM, tiles from a deepest-first counter), 16 warps.
-// Warp w serves the TMEM lane quadrant w mod 4 (one tile column, 32 voxels, a voxel
-// per lane) and the element slot w / 4 (elements 8s .. 8s+7 of every 32-element
-// chunk, one mma k-step).  Per tile the elements span the union of its voxels'
-// apertures; per bin only the chunks and k-steps that bin's apertures touch run
-// (the per-bin ranges come from a warp reduction along each column's segment lists),
-// with N = 16 ceil(transmit elements / 8).  Per bin and chunk the warps advance their
-// phasors p = e^{2 pi i k u} by p <- p conj(rho) in packed FP32x2 (rho = e^{2 pi i u}
-// kept in tensor memory, columns 256-511; exact re-anchoring every 32 bins and when a
-// chunk comes back into range) and write their A rows (fp16 hi/lo, 128-byte swizzle)
-// into a two-stage shared-memory ring.  The first warp through a stage issues the
-// item's B tiles (TMA, a 3-D map over [bin][row][column]); the last one in issues its
-// tcgen05.mma (M = 128, K = 16 per k-step: hi.lo and lo.hi first, then hi.hi) into
-// the single D accumulator and commits the stage and, after the bin's last chunk, D.
-// Once D is complete every thread reads its columns and adds n_k sum_t w_tx p_t Y_t
-// to its voxel (compensated sum); the next bin's first products are only issued
-// after every warp has passed that point, so D is free.  Waits sleep in the mbarrier
-// and give up after two seconds: the CTA then records ERR_TC_TIMEOUT, gives its
-// copies and products in flight time to land, frees its tensor memory and returns.
+// Kernel (persistent, one block per SM).  16 warps form A and take the dot products: warp w
+// serves lane quadrant w % 4 (a tile column, a voxel per thread) and element slot w / 4 (the
+// groups of 8 elements g with g % 4 = slot).  Per bin only the groups that the tile's apertures
+// touch run, with N = 16 (groups).  Per group a warp steps its phasors p <- p conj(rho) (kept in
+// tensor memory, 16 columns a group; exact every 32 bins and when a group comes back into
+// range), multiplies them with the receive window and writes the split rows to its slot's A tile
+// in shared memory.  Two threads issue the group's products (each for half of the transmit
+// elements), two copy its B tiles in turn.  When a bin's D is complete every warp adds n_k sum_t w_tx p_t Y_t of its groups to its
+// voxel (compensated sum).  The window of a voxel depends only on its column and the outermost
+// element of each side, so its values come from a table built with the plan; per bin and voxel
+// remain the table's rows and n_k, formed 4 bins ahead.
+//
+// What keeps the tensor cores busy is that a bin's products run beside the warps' work:
+// - up to 64 elements the phasors of two bins fit tensor memory: a bin's A is formed before the
+//   previous bin's dot products are taken;
+// - beyond, each slot forms the A of its first group before them (those phasors are stepped back
+//   for the dot product) and the others after them;
+// - bins of up to 64 elements use the two halves of D in turn, wider ones all of it.
+// A band of few tiles is split over the idle SMs.
+//
+// What bounds it: the latency of the chain from a bin's D over the dot products and the A of its
+// successor back to D (issue slots 47 %, tensor cores 26 % busy); 128 elements leave no room for
+// a second set of phasors, A tiles or accumulators that would cut it.
+// 128 elements, boxcar, 2-7 MHz, 400 x 400 voxels: 34.1 ms with 16 warps that wrote 32-element A
+// chunks, kept phasors in registers and searched segment lists; 18.8 ms here.  64 elements,
+// Hann, whole band, 151 x 187: 11.9 and 3.6 ms (windows from the table, two bins in flight, the
+// band in four ranges).  Fixed 16 KB B stages measured faster than a byte ring (20.3 and 23.7 ms
+// at the time), one copy per group and two issuing threads 1 % better than two and one.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
-#include <cmath>
+#include <mutex>
 
-#include "fnum_device.cuh"
-#include "fnum_internal.h"
-#include "fnum_tc_ptx.cuh"
+#include "fnum_tc_beam.cuh"
 
 namespace fnum {
 
@@ -57,533 +64,606 @@ namespace {
 
 using namespace tcx;
 
-constexpr int ST_M = 128;                            // voxels per tile = TMEM lanes = mma M
-constexpr int ST_KC = 32;                            // elements per chunk (64 fp16 = one 128-byte row)
-constexpr int ST_CMAX = 4;                           // chunks per bin: up to 128 elements
-constexpr int ST_EPT = 8;                            // elements per thread and chunk
-constexpr int ST_WARPS = 16;                         // 4 per TMEM lane quadrant
-constexpr int ST_THREADS = ST_WARPS * 32;
-constexpr int ST_STAGES = 2;
-constexpr int ST_A_PLANE = ST_M * 128;               // 16 KB
-constexpr int ST_B_PLANE = 2 * ST_KC * ST_CMAX * 128;   // up to 256 rows: 32 KB
-constexpr int ST_STAGE = 2 * ST_A_PLANE + 2 * ST_B_PLANE;
-constexpr int ST_SMEM = ST_STAGES * ST_STAGE + 1024;   // + alignment slack
-constexpr int ST_BOX_ROWS = 2 * ST_KC;               // B rows per TMA box: 32 transmit elements
-constexpr int ST_BOX_BYTES = ST_BOX_ROWS * 128;
-constexpr int ST_TB = 32;                            // bins between exact re-anchorings
-constexpr int ST_TMEM_COLS = 512;
-constexpr int ST_RHO_COL = 256;
+constexpr int ST_GMAX = 16;                 // element groups of 8: up to 128 elements
+constexpr int ST_TT = 4;                    // bins per aperture table (one per slot)
+constexpr int ST_NT = 4;                    // element ranges in flight (aperture tables: 2)
+constexpr int ST_NB = 8;                    // B stages at most
+constexpr int ST_A = 2 * P5_M * 32;         // a slot's A tile: hi, lo
+constexpr int ST_PH = 256;                  // TMEM: D below, the phasors (16 columns a group) from here
+constexpr int ST_NARROW = 128;              // D columns of a bin that fits half of D
 
-static_assert(ST_THREADS <= 1024, "block size");
-static_assert(ST_WARPS == 4 * (ST_KC / ST_EPT), "four slots per lane quadrant");
+struct StShared {
+  uint2 tab[2][ST_TT][P5_M];         // per bin and voxel: rows tx left, right, rx left, right (8 bits each), n_k
+  unsigned rng[ST_NT][ST_TT][4];     // per bin and column: element range lo | (0xffff - hi) << 16
+  float2 red[3][P5_M];
+  unsigned long long n_active, n_empty, n_exec;
+  int item, last;
+  int abort_flag;
+  uint32_t tmem;
+  uint64_t bars[4 + 4 + 2 * ST_NB + 4 + 2 * ST_NT];
+};
+
+// shared memory: StShared, A tiles, phasor steps, B stages
+__host__ __device__ inline int st_sh_bytes() { return ((int)sizeof(StShared) + 127) / 128 * 128; }
+__host__ __device__ inline int st_rho_bytes(int G) { return G * P5_M * 64; }
+__host__ __device__ inline int st_b_bytes(int G) { return G * 1024; }        // 64 N at N = 16 G
+constexpr int ST_SMEM_MAX = 232448;
+__host__ __device__ inline int st_stages(int G) {
+  const int n = (ST_SMEM_MAX - st_sh_bytes() - 4 * ST_A - st_rho_bytes(G)) / st_b_bytes(G);
+  return n < ST_NB ? n : ST_NB;
+}
 
 // ---------------------------------------------------------------------------
 // operands
 // ---------------------------------------------------------------------------
-// B planes [bin][n][kk] (n = 2t + p, kk = 2r + q, both < 2 nep) of X' scaled by the
-// power of two sigma; zero for t or r >= ne.  One block per (t, 32 receive elements,
-// 32 bins): the spectra are read along bins (coalesced) into shared memory and
-// written along receive elements.
-__global__ void __launch_bounds__(256) sa_tc_prep_kernel(const float2* __restrict__ X, int ne, int nep, int K,
+// B tiles of X' scaled by the power of two sigma, in the order the products read them: [bin][rx
+// group of 8][8 rows n][hi, lo][K half][n][8 fp16] (a group's row range is one copy), zero for t or r >= ne.  Row n holds transmit
+// element t = 8 (n / 16) + 2 (n % 16 / 4) + n % 2, real part (n % 4 < 2) or imaginary part of Y.
+// One block per (4 transmit elements, 32 receive elements, 8 bins): the spectra are read along
+// bins into shared memory and written as 32-byte row pairs.
+__global__ void __launch_bounds__(256) sa_tc_prep_kernel(const float2* __restrict__ X, int ne, int G, int K,
                                                          const float2* __restrict__ rot,
                                                          const unsigned* __restrict__ maxbits,
-                                                         __half2* __restrict__ bhi, __half2* __restrict__ blo) {
-  __shared__ float2 tile[32][33];
-  const int t = blockIdx.x, r0 = blockIdx.y * 32, k0 = blockIdx.z * 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int ri = w; ri < 32; ri += 8) {
-    const int r = r0 + ri, k = k0 + lane;
-    float2 x = make_float2(0.0f, 0.0f);
-    if (t < ne && r < ne && k < K) x = X[((size_t)t * ne + r) * K + k];
-    tile[ri][lane] = x;
+                                                         uint4* __restrict__ out) {
+  __shared__ float2 tile[4][32][9];
+  const int t0 = blockIdx.x * 4, r0 = blockIdx.y * 32, k0 = blockIdx.z * 8;
+  for (int i = threadIdx.x; i < 4 * 32 * 8; i += 256) {
+    const int kl = i & 7, rl = (i >> 3) & 31, tl = i >> 8;
+    const int t = t0 + tl, r = r0 + rl, k = k0 + kl;
+    tile[tl][rl][kl] = (t < ne && r < ne && k < K) ? X[((size_t)t * ne + r) * K + k] : make_float2(0.0f, 0.0f);
   }
   __syncthreads();
   const float sigma = tc_scale(*maxbits);
-  const size_t row = (size_t)nep;   // half2 per row: 2 nep fp16
-  for (int ki = w; ki < 32; ki += 8) {
-    const int k = k0 + ki, r = r0 + lane;
-    if (k >= K || r >= nep) continue;
-    float2 x = tile[lane][ki];
-    const float2 c = rot[k];
+  // thread: transmit element t, receive elements r .. r + 3, bin k
+  const int tl = threadIdx.x & 3, rq = (threadIdx.x >> 2) & 7, kl = threadIdx.x >> 5;
+  const int t = t0 + tl, r = r0 + 4 * rq, k = k0 + kl;
+  if (k >= K || r >= 8 * G) return;
+  const float2 c = rot[k];
+  unsigned h[2][4], l[2][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float2 x = tile[tl][4 * rq + i][kl];
     x = make_float2((x.x * c.x - x.y * c.y) * sigma, (x.x * c.y + x.y * c.x) * sigma);
-    // row 2t: (Re, -Im); row 2t + 1: (Im, Re)
-    const __half2 h0 = __floats2half2_rn(x.x, -x.y);
-    const __half2 h1 = __floats2half2_rn(x.y, x.x);
-    const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-    const __half2 l0 = __floats2half2_rn(x.x - f0.x, -x.y - f0.y);
-    const __half2 l1 = __floats2half2_rn(x.y - f1.x, x.x - f1.y);
-    const size_t i0 = ((size_t)k * 2 * nep + 2 * t) * row + r;
-    bhi[i0] = h0;
-    blo[i0] = l0;
-    bhi[i0 + row] = h1;
-    blo[i0 + row] = l1;
+    tc_split_mx(x.x, -x.y, h[0][i], l[0][i]);   // Re Y
+    tc_split_mx(x.y, x.x, h[1][i], l[1][i]);    // Im Y
+  }
+  const int kh = (r >> 2) & 1, n0 = 16 * (t >> 3) + 4 * ((t & 7) >> 1) + (t & 1);
+  uint4* o = out + ((size_t)k * G + (r >> 3)) * (size_t)(64 * G);   // a group: 2 G (8 rows) x 2 (hi, lo) x 16
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const int n = n0 + 2 * p;
+    uint4* q = o + (n >> 3) * 32 + kh * 8 + (n & 7);
+    q[0] = make_uint4(h[p][0], h[p][1], h[p][2], h[p][3]);
+    q[16] = make_uint4(l[p][0], l[p][1], l[p][2], l[p][3]);
   }
 }
 
 // ---------------------------------------------------------------------------
 // the beamformer
 // ---------------------------------------------------------------------------
-constexpr int ST_KMAX = 2048;       // bands up to this many bins get per-bin element ranges
-constexpr int ST_NONE = 1 << 20;    // empty range marker
+__device__ __forceinline__ unsigned st_range(const unsigned (&r)[4]) { return p5_uni(p5_join(r)); }
 
-struct StShared {
-  int ktop_tx[ST_M];
-  int ktop_rx[ST_M];
-  int nseg[ST_M];
-  float2 red[ST_WARPS / 4][ST_M];   // per element slot: the voxel's sum over the slot's elements
-  int ranges[4];
-  int tile;
-  int E_lo, E_hi, kt, nb;
-  unsigned long long n_active, n_empty;
-  uint32_t tmem;
-  int abort_flag;
-  int tma_cnt[2], mma_cnt[2];   // warps through each stage's item so far
-  uint64_t bars[7];   // a_full[2], b_full[2], s_empty[2], d_full
-  // per bin (relative to k_lb): the element range of the tile's apertures, tx and rx
-  int lo[ST_KMAX];
-  int hi[ST_KMAX];
-};
-
-// waits as long as no other thread has given up; records a timeout
-__device__ __forceinline__ bool st_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                        unsigned long long* err) {
-  if (mbar_test(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  for (;;) {
-    // sleep in the barrier (up to 20 us per test) instead of spinning on issue slots
-    if (mbar_test_sleep(bar, parity, 20000u)) return true;
-    if (*abort_flag) return false;
-    if (global_ns() - t0 > WAIT_NS) {
-      *abort_flag = 1;
-      atomicOr(err, ERR_TC_TIMEOUT);
-      return false;
+// Window values of a group's 8 elements by element pairs; false where every lane's are all 1.
+// BOX: the elements of an interval.  Otherwise the table's left and right rows, which hold
+// disjoint sides, so that only the group around the voxel's column needs both.
+template <bool BOX>
+__device__ __forceinline__ bool st_window(const float* wcol, unsigned row_l, unsigned row_r, int ne, int ne_pad, int g,
+                                          int emid, float2 (&w)[4]) {
+  const int e8 = 8 * g;
+  if constexpr (BOX) {
+    const int first = (int)row_l == ne ? emid : (int)row_l, last = (int)row_r == ne ? emid - 1 : (int)row_r;
+    if (__all_sync(0xffffffffu, first <= e8 && last >= e8 + 7)) return false;
+    const unsigned n = (unsigned)max(last - first + 1, 0), o = (unsigned)(e8 - first);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      w[i] = make_float2(o + 2u * i < n ? 1.0f : 0.0f, o + 2u * i + 1u < n ? 1.0f : 0.0f);
+  } else {
+    const unsigned row = e8 + 8 <= emid ? row_l : row_r;
+    const float4* r = reinterpret_cast<const float4*>(wcol + (row * (unsigned)ne_pad + (unsigned)e8));
+    float4 a = __ldg(r), b = __ldg(r + 1);
+    if (e8 < emid && e8 + 8 > emid) {
+      const float4* v = reinterpret_cast<const float4*>(wcol + (row_l * (unsigned)ne_pad + (unsigned)e8));
+      const float4 x = __ldg(v), y = __ldg(v + 1);
+      a = make_float4(a.x + x.x, a.y + x.y, a.z + x.z, a.w + x.w);
+      b = make_float4(b.x + y.x, b.y + y.y, b.z + y.z, b.w + y.w);
     }
+    w[0] = make_float2(a.x, a.y);
+    w[1] = make_float2(a.z, a.w);
+    w[2] = make_float2(b.x, b.y);
+    w[3] = make_float2(b.z, b.w);
+  }
+  return true;
+}
+
+// p <- w p
+__device__ __forceinline__ void st_weigh(const float2 (&w)[4], const float (&pv)[16], float (&v)[16]) {
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const float2 re = __fmul2_rn(w[x], make_float2(pv[4 * x], pv[4 * x + 1]));
+    const float2 im = __fmul2_rn(w[x], make_float2(pv[4 * x + 2], pv[4 * x + 3]));
+    v[4 * x] = re.x;
+    v[4 * x + 1] = re.y;
+    v[4 * x + 2] = im.x;
+    v[4 * x + 3] = im.y;
   }
 }
 
-// window weight of element e of a voxel (0 outside its aperture).  The aperture's
-// elements form the interval [a, b] = [min(i_lb, emid), max(i_ub, emid - 1)]: left of
-// emid from i_lb, right of it up to i_ub.
-template <int WIN>
-__device__ __forceinline__ float st_weight(const SADev& d, int e, int emid, int a, int b, float iLl, float iLr,
-                                           int ic, float par, float ipar) {
-  const bool in = e >= a && e <= b;
-  if (WIN == 0) return in ? 1.0f : 0.0f;
-  if (!in) return 0.0f;
-  const bool left = e < emid;
-  const dfl c = d.el_m[e], xm = d.col_m[ic];
-  const float dx = fabsf((c.x - xm.x) + (c.y - xm.y));
-  return win_t<WIN>(par, ipar, dx * (left ? iLl : iLr));
+// the phasor steps of a group, and p <- p rho
+__device__ __forceinline__ void st_rho(const float4* rhov, int g, float (&r4)[16]) {
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const float4 v = rhov[(4 * g + x) * P5_M];
+    r4[4 * x] = v.x;
+    r4[4 * x + 1] = v.y;
+    r4[4 * x + 2] = v.z;
+    r4[4 * x + 3] = v.w;
+  }
+}
+__device__ __forceinline__ void st_back(float (&pv)[16], const float (&rv)[16]) {
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float2 rr = make_float2(rv[4 * p], rv[4 * p + 1]), ri = make_float2(rv[4 * p + 2], rv[4 * p + 3]);
+    const float2 a = make_float2(pv[4 * p], pv[4 * p + 1]), m = make_float2(pv[4 * p + 2], pv[4 * p + 3]);
+    const float2 x = __ffma2_rn(p5_neg(m), ri, __fmul2_rn(a, rr));
+    const float2 y = __ffma2_rn(m, rr, __fmul2_rn(a, ri));
+    pv[4 * p] = x.x;
+    pv[4 * p + 1] = x.y;
+    pv[4 * p + 2] = y.x;
+    pv[4 * p + 3] = y.y;
+  }
 }
 
-__device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-
-template <int WT, int WR>
-__global__ void __launch_bounds__(ST_THREADS, 1)
-sa_tc_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo, const SADev d,
-             const unsigned* __restrict__ maxbits, float2* __restrict__ image, float* __restrict__ wtx_out,
-             float* __restrict__ wrx_out, int n_tiles_x, int n_tiles_z) {
-  extern __shared__ unsigned char dyn[];
-  __shared__ StShared sh;
-  const uint32_t raw = smem_u32(dyn);
-  const uint32_t base = (raw + 1023u) & ~1023u;   // the 128-byte swizzle wants 1024-byte tiles
-  unsigned char* gbase = dyn + (base - raw);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_tiles = n_tiles_x * n_tiles_z;
+// LAG: up to ST_GMAX / 2 groups, two bins' phasors in tensor memory; BOX: both windows boxcar
+template <bool LAG, bool BOX>
+__global__ void __launch_bounds__(P5_THREADS, 1)
+sa_tc_kernel(const SADev d, const uint4* __restrict__ Bt, const unsigned* __restrict__ maxbits,
+             float2* __restrict__ image, float* __restrict__ wtx_out, float* __restrict__ wrx_out) {
+  extern __shared__ __align__(128) unsigned char dyn[];
+  StShared& sh = *reinterpret_cast<StShared*>(dyn);
+  const int G = (d.ne + 7) >> 3;                    // element groups
+  const uint32_t NB = (uint32_t)st_stages(G), b_bytes = (uint32_t)st_b_bytes(G);
+  unsigned char* abuf = dyn + st_sh_bytes();
+  float4* rho = reinterpret_cast<float4*>(abuf + 4 * ST_A);
+  const uint32_t abase = smem_u32(abuf), bbase = smem_u32(rho) + (uint32_t)st_rho_bytes(G);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = (int)p5_uni((uint32_t)tid >> 5);
   volatile int* abort_flag = &sh.abort_flag;
   unsigned long long* err = &d.counters[2];
   const uint32_t bar0 = smem_u32(sh.bars);
-  auto a_full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
-  auto b_full = [&](int s) { return bar0 + 8u * (uint32_t)(2 + s); };
-  auto s_empty = [&](int s) { return bar0 + 8u * (uint32_t)(4 + s); };
-  const uint32_t d_full = bar0 + 48u;
-  const int per_bin = d.K <= ST_KMAX;
-  const int n_bins_tab = per_bin ? d.K : 0;
+  auto s_full = [&](uint32_t s) { return bar0 + 8u * s; };
+  auto s_empty = [&](uint32_t s) { return bar0 + 8u * (4u + s); };
+  auto d_full = [&](uint32_t s) { return bar0 + 8u * (8u + s); };
+  auto d_empty = [&](uint32_t s) { return bar0 + 8u * (10u + s); };
+  auto r_full = [&](uint32_t s) { return bar0 + 8u * (12u + s); };
+  auto r_empty = [&](uint32_t s) { return bar0 + 8u * (12u + ST_NT + s); };
+  auto b_full = [&](uint32_t s) { return bar0 + 8u * (12u + 2 * ST_NT + s); };
+  auto b_empty = [&](uint32_t s) { return bar0 + 8u * (12u + 2 * ST_NT + ST_NB + s); };
 
   if (tid == 0) {
-    for (int s = 0; s < ST_STAGES; ++s) {
-      mbar_init(a_full(s), ST_WARPS);
-      mbar_init(b_full(s), 1);
-      mbar_init(s_empty(s), 1);
-      sh.tma_cnt[s] = sh.mma_cnt[s] = 0;
+    for (int s = 0; s < 4; ++s) {
+      mbar_init(s_full(s), 4);
+      mbar_init(s_empty(s), 2);
     }
-    mbar_init(d_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(d_full(s), 2);
+      mbar_init(d_empty(s), P5_CW);
+    }
+    for (int s = 0; s < ST_NT; ++s) {
+      mbar_init(r_full(s), P5_CW);
+      mbar_init(r_empty(s), 4);
+    }
+    for (int s = 0; s < ST_NB; ++s) {
+      mbar_init(b_full(s), 1);
+      mbar_init(b_empty(s), 2);
+    }
     sh.abort_flag = 0;
-    sh.n_active = sh.n_empty = 0ull;
+    sh.n_active = sh.n_empty = sh.n_exec = 0ull;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async_smem();
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem)),
-                 "r"(ST_TMEM_COLS)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  const uint32_t tmem = sh.tmem;
+  const uint32_t tmem = p5_uni(sh.tmem);
+  const int ntx = (d.wt_nc + TILE_X - 1) / TILE_X, ntz = (d.nz + TILE_Z - 1) / TILE_Z;
+  const int n_items = ntx * ntz * d.split;
+  uint32_t nd = 0;                 // bins with products so far
+  uint32_t ns = 0;                 // aperture tables so far
+  const uint32_t lead = lane == 0 ? 1u : 0u;
 
-  const float sigma = tc_scale(*maxbits);
-  const float ipt = (d.wtx_par > 0.0f) ? 1.0f / d.wtx_par : 0.0f;
-  const float ipr = (d.wrx_par > 0.0f) ? 1.0f / d.wrx_par : 0.0f;
-  // the warp's TMEM lane quadrant (tile column) and element slot
-  const int q = warp & 3, slot = warp >> 2;
-  const int vb = 32 * q + lane;
-  const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
-  const uint32_t row_off = (uint32_t)((vb >> 3) * 1024 + (vb & 7) * 128);
-  const uint32_t ch0 = (uint32_t)(((2 * slot) ^ (vb & 7)) << 4), ch1 = (uint32_t)(((2 * slot + 1) ^ (vb & 7)) << 4);
-  // running counts of (bin, chunk) items and of bins with products, the same in every warp
-  uint32_t it = 0, bn = 0;
-  unsigned long long n_exec = 0;
-
-  for (;;) {
-    if (tid == 0) sh.tile = (int)atomicAdd(&d.counters[3], 1ull);
-    for (int e = tid; e < ST_M; e += ST_THREADS) sh.ktop_tx[e] = sh.ktop_rx[e] = -1;
-    if (tid == 0) {
-      sh.ranges[0] = sh.ranges[2] = d.ne;
-      sh.ranges[1] = sh.ranges[3] = -1;
-    }
-    __syncthreads();
-    const int tile = sh.tile;
-    if (tile >= n_tiles || *abort_flag) break;
-    int tx_, tz_;
-    tile_coords(tile, n_tiles_x, n_tiles_z, tx_, tz_);
-    const int i = tx_ * TILE_X + q, j = tz_ * TILE_Z + lane;
-    const bool vvalid = (i < d.nx) && (j < d.nz);
-    const int ic = min(i, d.nx - 1), jc = min(j, d.nz - 1);
-    int4* seg = d.seg + ((size_t)blockIdx.x * ST_M + vb) * (size_t)d.seg_cap * SA_SEG_INT4;
-    const int emid = d.col_emid[ic];
-    for (int kk = tid; kk < n_bins_tab; kk += ST_THREADS) {
-      sh.lo[kk] = ST_NONE;
-      sh.hi[kk] = -1;
-    }
-    if (warp < 4) {
-      float Wt, Wr;
-      unsigned long long na = 0, nm = 0;
-      sh.nseg[vb] = sa_build_segments(d, ic, jc, vvalid, seg, sh.ktop_tx, sh.ktop_rx, sh.ranges, Wt, Wr, na, nm);
-      atomicAdd(&sh.n_active, na);
-      atomicAdd(&sh.n_empty, nm);
-      if (vvalid) {
-        if (wtx_out) wtx_out[(size_t)ic * d.nz + jc] = Wt;
-        if (wrx_out) wrx_out[(size_t)ic * d.nz + jc] = Wr;
-      }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      const int lo = min(sh.ranges[0], sh.ranges[2]), hi = max(sh.ranges[1], sh.ranges[3]);
-      int kt = -1;
-      if (lo <= hi)
-        for (int e = lo; e <= min(hi, d.ne - 1); ++e) kt = max(kt, max(sh.ktop_tx[e], sh.ktop_rx[e]));
-      sh.E_lo = lo;
-      sh.E_hi = hi;
-      sh.kt = kt;
-      sh.nb = (lo <= hi && kt >= d.k_lb) ? kt - d.k_lb + 1 : 0;
-    }
-    __syncthreads();
-    const int E_lo = sh.E_lo, E_hi = sh.E_hi, kt = sh.kt, nb = sh.nb;
-    const int E0 = E_lo & ~7;   // the threads' elements: E0 + 32 c + 8 slot + i
-    const int ns = sh.nseg[vb];
-    // per bin, the element range of the tile's apertures: a reduction over each column's
-    // voxels along their segment lists, then over the four columns
-    if (per_bin && nb > 0 && warp < 4) {
-      int sidx = (ns > 0) ? sa_seg_find(seg, ns, kt) : 0;
-      int nxt = (ns > 0) ? seg[min(sidx + 1, ns)].x : -1;
-      int a = ST_NONE, b = -1;
-      auto rng = [&]() {
-        a = ST_NONE;
-        b = -1;
-        if (ns == 0) return;
-        const int4 cur = seg[sidx];
-        if (cur.w == 0) return;   // an empty aperture: no term
-        a = min(min(code_ilb(cur.y), code_ilb(cur.z)), emid);
-        b = max(max(code_iub(cur.y), code_iub(cur.z)), emid - 1);
-      };
-      rng();
-      for (int k = kt; k >= d.k_lb; --k) {
-        if (k == nxt) {
-          ++sidx;
-          nxt = seg[min(sidx + 1, ns)].x;
-          rng();
-        }
-        const int mn = __reduce_min_sync(0xffffffffu, a), mx = __reduce_max_sync(0xffffffffu, b);
-        if (lane == 0 && mn <= mx) {
-          atomicMin(&sh.lo[k - d.k_lb], mn);
-          atomicMax(&sh.hi[k - d.k_lb], mx);
-        }
-      }
-    }
-    __syncthreads();
-    float2 acc = make_float2(0.0f, 0.0f), comp = make_float2(0.0f, 0.0f);
-    if (nb > 0) {
-      auto u_of = [&](int e) {
-        return df_sqrt(df_add(df_sqr(df_sub(d.el_u[min(e, d.ne - 1)], d.col_u[ic])), d.row_u2[jc]));
-      };
-      // rho = e^{2 pi i u} of the thread's elements into tensor memory, by element pairs
-      // {Re rho_2j, Re rho_2j+1, Im rho_2j, Im rho_2j+1} (the packed recurrence's operands)
-      for (int c = 0; c * ST_KC <= E_hi - E0; ++c) {
-        float rv[16];
-#pragma unroll
-        for (int k2 = 0; k2 < ST_EPT; ++k2) {
-          const float2 r = cis_ku(1, u_of(E0 + ST_KC * c + ST_EPT * slot + k2));
-          rv[4 * (k2 >> 1) + (k2 & 1)] = r.x;
-          rv[4 * (k2 >> 1) + 2 + (k2 & 1)] = r.y;
-        }
-        tmem_st16(tl + (uint32_t)(ST_RHO_COL + 2 * ST_KC * c + 2 * ST_EPT * slot), rv);
-      }
-      tmem_wait_st();
-      // the segment in effect: its apertures, normaliser and (other windows) half-widths
-      // (the next entry is loaded a boundary ahead, so its latency hides behind whole bins)
-      int sidx = (ns > 0) ? sa_seg_find(seg, ns, kt) : 0;
-      int4 nxt = (ns > 0) ? seg[min(sidx + 1, ns)] : make_int4(-1, 0, 0, 0);
-      int ta = 0, tb = -1, ra = 0, rb = -1;
-      float nrm = 0.0f, tLl = 0.0f, tLr = 0.0f, rLl = 0.0f, rLr = 0.0f;
-      auto derive = [&](const int4 cur) {
-        const int tlb = code_ilb(cur.y), tub = code_iub(cur.y), rlb = code_ilb(cur.z), rub = code_iub(cur.z);
-        ta = min(tlb, emid);
-        tb = max(tub, emid - 1);
-        ra = min(rlb, emid);
-        rb = max(rub, emid - 1);
-        nrm = __int_as_float(cur.w);
-        if (WT != 0 || WR != 0) {
-          const dfl xm = d.col_m[ic];
-          if (WT != 0) {
-            tLl = (tlb < d.ne) ? inv_half_width(d.el_lb, d.el_ub, xm, true, tlb, tub) : 0.0f;
-            tLr = (tub >= 0) ? inv_half_width(d.el_lb, d.el_ub, xm, false, tlb, tub) : 0.0f;
+  if (warp >= P5_CW) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P5_REGS_I));
+    const int role = warp - P5_CW;       // 0, 1: products of the first, second half of the transmit elements; 2, 3: copies
+    uint32_t st = 0, st_ph = 0;          // B stage and its phase
+    uint32_t turn = 0;                   // the copying threads take groups in turn
+    uint32_t a_ph = 0;                   // phases of the slots' A tiles (bit per slot)
+    bool prev_wide = false;
+    for (;;) {
+      __syncthreads();
+      const int item = sh.item;
+      if (item < 0) break;
+      const int part = item % d.split;
+      const int kt = d.k_ub - part * d.split_bins;
+      const int nb = min(d.split_bins, kt - d.k_lb + 1);
+      if (lane == 0) {
+        unsigned long long exec = 0;
+        bool ok = true;
+        for (int b = 0; b < nb && ok; ++b) {
+          const uint32_t ri = ns % ST_NT;
+          if (b % ST_TT == 0) ok = p5_wait(r_full(ri), (ns / ST_NT) & 1u, 0u, abort_flag, err);
+          const unsigned r = p5_join(sh.rng[ri][b % ST_TT]);
+          // the last use of this table's ranges
+          if (b % ST_TT == ST_TT - 1 || b == nb - 1) {
+            mbar_arrive(r_empty(ri));
+            ++ns;
           }
-          if (WR != 0) {
-            rLl = (rlb < d.ne) ? inv_half_width(d.el_lb, d.el_ub, xm, true, rlb, rub) : 0.0f;
-            rLr = (rub >= 0) ? inv_half_width(d.el_lb, d.el_ub, xm, false, rlb, rub) : 0.0f;
-          }
-        }
-      };
-      derive((ns > 0) ? seg[sidx] : make_int4(-1, seg_code(d.ne, -1), seg_code(d.ne, -1), 0));
-      // phasors by element pairs: pr[c][j] = {Re p_2j, Re p_2j+1}, pm[c][j] = {Im p_2j, Im p_2j+1}
-      float2 pr[ST_CMAX][ST_EPT / 2], pm[ST_CMAX][ST_EPT / 2];
-#pragma unroll
-      for (int c = 0; c < ST_CMAX; ++c)
-#pragma unroll
-        for (int j2 = 0; j2 < ST_EPT / 2; ++j2) pr[c][j2] = pm[c][j2] = make_float2(0.0f, 0.0f);
-      // per chunk: p holds the phasors of the previous bin (else the next use re-anchors)
-      unsigned live = 0u;
-      bool ok = true;
-      for (int b = 0; b < nb && ok; ++b) {
-        const int k = kt - b;
-        if (k == nxt.x) {
-          const int4 cur = nxt;
-          ++sidx;
-          nxt = seg[min(sidx + 1, ns)];
-          derive(cur);
-        }
-        int lo = E_lo, hi = E_hi;
-        if (per_bin) {
-          lo = sh.lo[k - d.k_lb];
-          hi = sh.hi[k - d.k_lb];
-        }
-        if (lo > hi) {   // no aperture in the tile at this bin
-          live = 0u;
-          continue;
-        }
-        // this bin's chunks c_lo..c_hi; transmit rows from E0b (D column 2 (e - E0b))
-        const int E0b = lo & ~7;
-        const int c_lo = (lo - E0) >> 5, c_hi = (hi - E0) >> 5;
-        const int nN = 16 * ((hi - E0b + 8) >> 3);
-        const uint32_t idesc = idesc_f16(ST_M, nN);
-        const int nbox = (nN + ST_BOX_ROWS - 1) / ST_BOX_ROWS;
-        const uint32_t box_bytes = (uint32_t)(2 * nbox * ST_BOX_BYTES);
-        const bool anchor = (b % ST_TB) == 0;
-        unsigned nlive = 0u;
-        int n_items = 0;
-#pragma unroll
-        for (int c = 0; c < ST_CMAX; ++c) {
-          if (c >= c_lo && c <= c_hi) {
-            const int g0 = E0 + ST_KC * c;
-            const int s_lo = max(0, (lo - g0) >> 3), s_hi = min(ST_KC / ST_EPT - 1, (hi - g0) >> 3);
-            const bool mine = slot >= s_lo && slot <= s_hi;
-            const int eb = g0 + ST_EPT * slot;
-            const bool exact = anchor || !(live & (1u << c));
-            const int st = (int)(it & 1u);
-            const uint32_t ph = (it >> 1) & 1u;
-            unsigned char* ahi = gbase + st * ST_STAGE;
-            unsigned char* alo = ahi + ST_A_PLANE;
-            // two halves of 4 elements: phasors, A values, then (once the stage is free) the stores
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint32_t hq[4], lq[4];
-              if (mine) {
-                if (exact) {
-#pragma unroll
-                  for (int jj = 0; jj < 2; ++jj) {
-                    const int j2 = 2 * h + jj;
-                    const float2 z0 = cis_ku(k, u_of(eb + 2 * j2)), z1 = cis_ku(k, u_of(eb + 2 * j2 + 1));
-                    pr[c][j2] = make_float2(z0.x, z1.x);
-                    pm[c][j2] = make_float2(z0.y, z1.y);
-                  }
-                } else {
-                  // p <- p conj(rho), two elements per packed FP32 instruction
-                  float rv[8];
-                  tmem_ld8_nowait(tl + (uint32_t)(ST_RHO_COL + 2 * ST_KC * c + 2 * ST_EPT * slot + 8 * h), rv);
-                  tmem_wait_ld();
-#pragma unroll
-                  for (int jj = 0; jj < 2; ++jj) {
-                    const int j2 = 2 * h + jj;
-                    const float2 rr = make_float2(rv[4 * jj], rv[4 * jj + 1]);
-                    const float2 ri = make_float2(rv[4 * jj + 2], rv[4 * jj + 3]);
-                    const float2 a = pr[c][j2], m = pm[c][j2];
-                    const float2 t = __fmul2_rn(a, ri);
-                    pr[c][j2] = __ffma2_rn(m, ri, __fmul2_rn(a, rr));
-                    pm[c][j2] = __ffma2_rn(m, rr, make_float2(-t.x, -t.y));
-                  }
-                }
-#pragma unroll
-                for (int kq = 0; kq < 4; ++kq) {
-                  const int k2 = 4 * h + kq;
-                  const float w = st_weight<WR>(d, eb + k2, emid, ra, rb, rLl, rLr, ic, d.wrx_par, ipr);
-                  const float px = (k2 & 1) ? pr[c][k2 >> 1].y : pr[c][k2 >> 1].x;
-                  const float py = (k2 & 1) ? pm[c][k2 >> 1].y : pm[c][k2 >> 1].x;
-                  const float br = w * px, bi = w * py;
-                  const __half2 hh = __floats2half2_rn(br, bi);
-                  const float2 f = __half22float2(hh);
-                  hq[kq] = h2u(hh);
-                  lq[kq] = h2u(__floats2half2_rn(br - f.x, bi - f.y));
-                }
-              }
-              if (h == 0) {
-                // the stage is free once the products of the item two back have read it
-                ok = __all_sync(0xffffffffu, st_wait(s_empty(st), ph ^ 1u, abort_flag, err));
+          if (r == 0xffffffffu) continue;
+          const int g_lo = (int)(r & 0xffffu) >> 3, g_hi = (0xffff - (int)(r >> 16)) >> 3;
+          const int ng = g_hi - g_lo + 1;
+          if (role >= 2) {
+            // per group: rows 16 g_lo .. 16 g_hi + 15
+            const uint4* src = Bt + ((size_t)(kt - b - d.k_lb) * G + g_lo) * (size_t)(64 * G) + 64 * g_lo;
+            for (int g = g_lo; g <= g_hi; ++g, src += 64 * G) {
+              if (turn == ((uint32_t)role & 1u)) {
+                ok = p5_wait(b_empty(st), st_ph ^ 1u, 0u, abort_flag, err);
                 if (!ok) break;
-                if (lane == 0) {
-                  // the first warp through issues the item's B tiles, the last one resets the count
-                  const int o = atomicAdd(&sh.tma_cnt[st], 1);
-                  if (o == 0) {
-                    const uint32_t bh = base + (uint32_t)(st * ST_STAGE + 2 * ST_A_PLANE);
-                    const uint32_t bl = bh + ST_B_PLANE;
-                    mbar_expect_tx(b_full(st), box_bytes);
-                    const int x = 2 * g0, z = k - d.k_lb;
-                    for (int jj = 0; jj < nbox; ++jj) {
-                      const int y = 2 * E0b + ST_BOX_ROWS * jj;
-                      tma_load_3d(bh + (uint32_t)(jj * ST_BOX_BYTES), &tm_hi, x, y, z, b_full(st));
-                      tma_load_3d(bl + (uint32_t)(jj * ST_BOX_BYTES), &tm_lo, x, y, z, b_full(st));
-                    }
-                  } else if (o == ST_WARPS - 1) {
-                    sh.tma_cnt[st] = 0;
-                  }
+                mbar_expect_tx(b_full(st), 1024u * (uint32_t)ng);
+                bulk_load(bbase + st * b_bytes, src, 1024u * (uint32_t)ng, b_full(st));
+              }
+              turn ^= 1u;
+              if (++st == NB) {
+                st = 0;
+                st_ph ^= 1u;
+              }
+            }
+            if (role == 2) exec += (unsigned long long)P5_M * 64 * ng * ng;
+          } else {
+            // D: a half in turn for narrow bins; the bin before it must have been read where the two overlap
+            const bool wide = 16 * ng > ST_NARROW;
+            const uint32_t last = (wide || prev_wide) ? 1u : 2u;   // the bin read before this one writes: nd - last
+            prev_wide = wide;
+            uint32_t ask_a = p5_ask(s_full((uint32_t)g_lo & 3u), (a_ph >> (g_lo & 3)) & 1u);
+            uint32_t ask_b = p5_ask(b_full(st), st_ph);
+            // this thread's rows
+            const int n0 = (ng + 1) >> 1;
+            const uint32_t row0 = role ? (uint32_t)n0 : 0u, n = 16u * (uint32_t)(role ? ng - n0 : n0);
+            const uint32_t dcol = tmem + (wide ? 0u : (nd & 1u) * ST_NARROW) + 16u * row0;
+            const uint32_t idesc = idesc_f16(P5_M, (int)n);
+            constexpr uint64_t HA = smem_desc_plain_hi(256), HB = smem_desc_plain_hi(512);
+            const uint32_t b0 = (uint32_t)smem_desc_plain(bbase, 128, 512) + 64u * row0;
+            const uint32_t a0 = (uint32_t)smem_desc_plain(abase, 128, 256);
+            if (nd >= last)
+              ok = p5_wait(d_empty((nd - last) & 1u), ((nd - last) >> 1) & 1u, 0u, abort_flag, err);
+            uint32_t accum = 0u;
+            for (int g = g_lo; g <= g_hi; ++g) {
+              const uint32_t sl = (uint32_t)g & 3u;
+              p5_wait(b_full(st), st_ph, ask_b, abort_flag, err);
+              p5_wait(s_full(sl), (a_ph >> sl) & 1u, ask_a, abort_flag, err);
+              const uint32_t bd = b0 + st * (b_bytes >> 4), ah = a0 + sl * (ST_A >> 4);
+              const uint32_t be = b_empty(st), nx = (sl + 1u) & 3u;
+              a_ph ^= 1u << sl;
+              if (++st == NB) {
+                st = 0;
+                st_ph ^= 1u;
+              }
+              fence_after_sync();
+              if (n) {
+                // the small cross products first, so that fewer steps round a full-size sum
+                mma_f16(dcol, HA | (uint64_t)ah, HB | (uint64_t)(bd + 16u), idesc, accum);
+                mma_f16(dcol, HA | (uint64_t)(ah + (ST_A >> 5)), HB | (uint64_t)bd, idesc, 1u);
+                mma_f16(dcol, HA | (uint64_t)ah, HB | (uint64_t)bd, idesc, 1u);
+              }
+              accum = 1u;
+              mma_commit(s_empty(sl));
+              mma_commit(be);
+              ask_b = p5_ask(b_full(st), st_ph);
+              ask_a = p5_ask(s_full(nx), (a_ph >> nx) & 1u);
+            }
+            mma_commit(d_full(nd & 1u));
+            ok = ok && !*abort_flag;
+          }
+          ++nd;
+        }
+        if (role == 2) sh.n_exec += exec;
+      }
+      __syncwarp();
+      __syncthreads();
+    }
+  } else {
+    // ----------------------------------------------------------------------------------- A and D
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P5_REGS_C));
+    const int q = warp & 3, slot = warp >> 2;         // lane quadrant (tile column), slot
+    const int vb = 32 * q + lane;
+    const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+    float4* us = d.u_scr + (size_t)blockIdx.x * (size_t)(P5_M * 4 * ST_GMAX) + vb;
+    const uint32_t sf = s_full((uint32_t)slot), se = s_empty((uint32_t)slot);
+    unsigned char* arow = abuf + slot * ST_A + (vb >> 3) * 256 + (vb & 7) * 16;
+    const float4* rhov = rho + vb;
+    const float inv_sigma = 1.0f / tc_scale(*maxbits);
+    const int ne = d.ne;
+    uint32_t a_ph = 0;                                // phase of the slot's A tile
+    for (;;) {
+      if (tid == 0) {
+        const int t = *abort_flag ? n_items : (int)atomicAdd(&d.counters[3], 1ull);
+        sh.item = t < n_items ? t : -1;
+      }
+      __syncthreads();
+      const int item = sh.item;
+      if (item < 0) break;
+      const int tile = item / d.split, part = item - tile * d.split;
+      int tx, tz;
+      tile_coords(tile, ntx, ntz, tx, tz);
+      const int cw = tx * TILE_X + q;                       // column within the window tables' slab
+      const int j = tz * TILE_Z + lane;
+      const bool valid = (cw < d.wt_nc) && (j < d.nz);
+      const int cc = min(cw, d.wt_nc - 1), ic = d.wt_c0 + cc, jc = min(j, d.nz - 1);
+      const size_t vox = (size_t)ic * d.nz + jc;
+      const int kt = d.k_ub - part * d.split_bins;
+      const int nb = min(d.split_bins, kt - d.k_lb + 1);
+      const int emid = (int)p5_uni((uint32_t)d.col_emid[ic]);
+      const float* wt_col = d.w_tab[0] + (size_t)cc * (size_t)(ne + 1) * d.ne_pad;
+      const float* wr_col = d.w_tab[1] + (size_t)cc * (size_t)(ne + 1) * d.ne_pad;
+      unsigned c_act = 0, c_emp = 0;
+      // Aperture table of stretch s: per bin and voxel the rows of the window tables and n_k, per bin and column
+      // the element range; this warp takes its column's bin `slot`.
+      auto build = [&](int s) {
+        const uint32_t tbuf = (ns + (uint32_t)s) & 1u, ri = (ns + (uint32_t)s) % ST_NT;
+        const uint32_t rp = (((ns + (uint32_t)s) / ST_NT) & 1u) ^ 1u;
+        const uint32_t ask = p5_ask(r_empty(ri), rp);
+        const dfl xp = d.col_p[ic], zp = d.row_p[jc];
+        const int b = s * ST_TT + slot;
+        const int kk = max(kt - b - d.k_lb, 0);
+        int tlb, tub, rlb, rub;
+        p5_aperture(xp, zp, d.gtx[kk], ne, tlb, tub);
+        rlb = tlb;
+        rub = tub;
+        if (!d.Xs) p5_aperture(xp, zp, d.grx[kk], ne, rlb, rub);
+        // a side without elements takes the zero row
+        const int t_l = tlb < emid ? tlb : ne, t_r = tub >= emid ? tub : ne;
+        const int r_l = rlb < emid ? rlb : ne, r_r = rub >= emid ? rub : ne;
+        const float* s0 = d.w_sum[0] + (size_t)cc * (size_t)(ne + 1);
+        const float* s1 = d.w_sum[1] + (size_t)cc * (size_t)(ne + 1);
+        const float Wt = __ldg(s0 + t_l) + __ldg(s0 + t_r);
+        const float Wr = d.Xs ? Wt : __ldg(s1 + r_l) + __ldg(s1 + r_r);
+        const float it = Wt > 0.0f ? (d.norm_tx ? __frcp_rn(Wt) : 1.0f) : 0.0f;
+        const float ir = Wr > 0.0f ? (d.norm_rx ? __frcp_rn(Wr) : 1.0f) : 0.0f;
+        const int t_n = max(tub, emid - 1) - min(tlb, emid) + 1, r_n = max(rub, emid - 1) - min(rlb, emid) + 1;
+        const bool in = valid && b < nb;
+        const bool act = in && Wt > 0.0f && Wr > 0.0f && t_n > 0 && r_n > 0;
+        if (in) {
+          if (act) c_act += (unsigned)(t_n * r_n); else ++c_emp;
+          if (kk == d.K - 1) {
+            if (wtx_out) wtx_out[vox] = Wt;
+            if (wrx_out) wrx_out[vox] = Wr;
+          }
+        }
+        const int lo = act ? min(min(tlb, rlb), emid) : 0xffff, hi = act ? max(max(tub, rub), emid - 1) : -1;
+        p5_wait(r_empty(ri), rp, ask, abort_flag, err);
+        sh.tab[tbuf][slot][vb] = make_uint2((unsigned)t_l | (unsigned)t_r << 8 | (unsigned)r_l << 16 | (unsigned)r_r << 24,
+                                            __float_as_uint(act ? it * ir : 0.0f));
+        const unsigned mn = __reduce_min_sync(0xffffffffu, (unsigned)lo);
+        const int mx = __reduce_max_sync(0xffffffffu, hi);
+        if (lead) sh.rng[ri][slot][q] = mx < 0 ? 0xffffffffu : (mn | ((unsigned)(0xffff - mx) << 16));
+        __syncwarp();
+        mbar_arrive_if(lead, r_full(ri));
+      };
+      build(0);
+      // phasor steps rho = e^{2 pi i u} into shared memory, by element pairs {Re, Re, Im, Im}; the
+      // delays u to scratch for the exact anchors
+#pragma unroll 1
+      for (int g = slot; g < G; g += 4) {
+#pragma unroll
+        for (int j2 = 0; j2 < 4; ++j2) {
+          dfl u[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int e = min(8 * g + 2 * j2 + h, ne - 1);
+            u[h] = df_sqrt(df_add(df_sqr(df_sub(d.el_u[e], d.col_u[ic])), d.row_u2[jc]));
+          }
+          float2 r, m;
+          p5_cis2(1.0f, make_float2(u[0].x, u[1].x), make_float2(u[0].y, u[1].y), r, m);
+          rho[(4 * g + j2) * P5_M + vb] = make_float4(r.x, r.y, m.x, m.y);
+          us[(size_t)(4 * g + j2) * P5_M] = make_float4(u[0].x, u[1].x, u[0].y, u[1].y);
+        }
+      }
+      float2 acc = make_float2(0.0f, 0.0f), comp = make_float2(0.0f, 0.0f);
+      unsigned live = 0u;                 // groups whose phasors belong to the previous bin
+      // the bin whose products are under way: its groups, transmit rows and n_k
+      unsigned p_mask = 0u, p_rows = 0u;
+      int p_glo = 0;
+      float p_nrm = 0.0f;
+      bool p_wide = false;
+#pragma unroll 1
+      for (int b = 0; b <= nb; ++b) {
+        unsigned mask = 0u;
+        uint2 te = make_uint2(0u, 0u);
+        int g_lo = 0, g_hi = -1;
+        if (b < nb) {
+          const int s = b / ST_TT, t = b % ST_TT;
+          if (t == 0) {
+            // table s is complete, and no warp reads the one before it any more
+            p5_bar();
+            if (b + ST_TT < nb) build(s + 1);
+          }
+          const unsigned r = st_range(sh.rng[(ns + (uint32_t)s) % ST_NT][t]);
+          if (b % 32 == 0) live = 0u;     // exact phasors
+          if (r == 0xffffffffu) {         // no aperture in the tile at this bin
+            live = 0u;
+            continue;
+          }
+          te = sh.tab[(ns + (uint32_t)s) & 1u][t][vb];
+          g_lo = (int)(r & 0xffffu) >> 3;
+          g_hi = (0xffff - (int)(r >> 16)) >> 3;
+          mask = (2u << g_hi) - (1u << g_lo);
+        }
+        const bool wide = 16 * (g_hi - g_lo + 1) > ST_NARROW;
+        const unsigned exact = mask & ~live;
+        const uint32_t cur = nd, prv = nd - 1u;          // counts of this bin and of the one under way
+        const uint32_t ph_n = tl + ST_PH + (LAG ? (cur & 1u) * 128u : 0u);
+        const uint32_t ph_o = tl + ST_PH + (LAG ? (prv & 1u) * 128u : 0u);
+        const uint32_t td = tl + (p_wide ? 0u : (prv & 1u) * ST_NARROW);
+        float2 sx = make_float2(0.0f, 0.0f), sy = make_float2(0.0f, 0.0f);
+        const unsigned ms = mask & (0x1111u << slot);
+        const unsigned head = LAG ? ms : ms & (0u - ms);
+#pragma unroll 1
+        for (int pass = 0; pass < (LAG ? 2 : 3); ++pass) {
+          // A of the slot's first group (LAG: of all), the previous bin's dot products, the other groups' A
+          const unsigned dots = pass == 1 ? p_mask : 0u;
+          const unsigned gens = pass == 0 ? head : (pass == 2 ? ms & ~head : 0u);
+          if (dots) {
+            p5_wait(d_full(prv & 1u), (prv >> 1) & 1u, 0u, abort_flag, err);
+            fence_after_sync();
+          }
+          const unsigned mine = (dots | gens) & (0x1111u << slot);
+#pragma unroll 1
+          for (unsigned m = mine; m; m &= m - 1u) {
+            const int g = __ffs(m) - 1;
+            if ((dots >> g) & 1u) {
+              float y[16], p[16];
+              tmem_ld16_nowait(td + (uint32_t)(16 * (g - p_glo)), y);
+              tmem_ld16_nowait(ph_o + (uint32_t)(16 * g), p);
+              float2 w[4];
+              const bool weigh = st_window<BOX>(wt_col, p_rows & 0xffu, (p_rows >> 8) & 0xffu, ne, d.ne_pad, g, emid, w);
+              tmem_wait_ld();
+              if (!LAG && ((head >> g) & 1u)) {   // its phasors are this bin's
+
+                float r4[16];
+                st_rho(rhov, g, r4);
+                st_back(p, r4);
+              }
+              if (weigh) st_weigh(w, p, p);
+#pragma unroll
+              for (int x = 0; x < 4; ++x) {
+                const float2 ar = make_float2(p[4 * x], p[4 * x + 1]), ai = make_float2(p[4 * x + 2], p[4 * x + 3]);
+                const float2 yr = make_float2(y[4 * x], y[4 * x + 1]), yi = make_float2(y[4 * x + 2], y[4 * x + 3]);
+                sx = __ffma2_rn(ar, yr, __ffma2_rn(p5_neg(ai), yi, sx));
+                sy = __ffma2_rn(ar, yi, __ffma2_rn(ai, yr, sy));
+              }
+            }
+            if ((gens >> g) & 1u) {
+              const bool fresh = (exact >> g) & 1u;
+              float p[16];
+              if (!fresh) tmem_ld16_nowait(ph_o + (uint32_t)(16 * g), p);
+              const uint32_t ask_a = p5_ask(se, a_ph ^ 1u);
+              float2 w[4];
+              const bool weigh = st_window<BOX>(wr_col, (te.x >> 16) & 0xffu, te.x >> 24, ne, d.ne_pad, g, emid, w);
+              if (fresh) {
+                const float kf = (float)(kt - b);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                  const float4 u = us[(size_t)(4 * g + x) * P5_M];
+                  float2 re, im;
+                  p5_cis2(kf, make_float2(u.x, u.y), make_float2(u.z, u.w), re, im);
+                  p[4 * x] = re.x;
+                  p[4 * x + 1] = re.y;
+                  p[4 * x + 2] = im.x;
+                  p[4 * x + 3] = im.y;
                 }
+              } else {
+                float r4[16];
+                st_rho(rhov, g, r4);
+                tmem_wait_ld();
+                p5_rotate(p, r4);
               }
-              if (mine) {
-                const uint32_t chh = h ? ch1 : ch0;
-                *reinterpret_cast<uint4*>(ahi + row_off + chh) = make_uint4(hq[0], hq[1], hq[2], hq[3]);
-                *reinterpret_cast<uint4*>(alo + row_off + chh) = make_uint4(lq[0], lq[1], lq[2], lq[3]);
+              tmem_st16(ph_n + (uint32_t)(16 * g), p);
+              uint32_t h[8], l[8];
+              if (weigh) st_weigh(w, p, p);
+#pragma unroll
+              for (int x = 0; x < 4; ++x) {
+                tc_split_mx(p[4 * x], p[4 * x + 2], h[2 * x], l[2 * x]);
+                tc_split_mx(p[4 * x + 1], p[4 * x + 3], h[2 * x + 1], l[2 * x + 1]);
               }
-            }
-            if (!ok) break;
-            if (mine) {
-              nlive |= 1u << c;
+              // the slot's A tile is free once the products that read it last are complete
+              p5_wait(se, a_ph ^ 1u, ask_a, abort_flag, err);
+              uint4* o = reinterpret_cast<uint4*>(arow);
+              o[0] = make_uint4(h[0], h[1], h[2], h[3]);
+              o[8] = make_uint4(h[4], h[5], h[6], h[7]);
+              o[ST_A / 32] = make_uint4(l[0], l[1], l[2], l[3]);
+              o[ST_A / 32 + 8] = make_uint4(l[4], l[5], l[6], l[7]);
               fence_proxy_async_smem();
+              __syncwarp();
+              mbar_arrive_if(lead, sf);
+              a_ph ^= 1u;
+              tmem_wait_st();
             }
+          }
+          if (dots) {
             fence_before_sync();
             __syncwarp();
-            if (lane == 0) {
-              mbar_arrive(a_full(st));
-              // the last warp in issues the item's products for the chunk's live k-steps (all A
-              // rows are written, and for the bin's first chunk every warp has read the previous
-              // bin's D)
-              const int o = atomicAdd(&sh.mma_cnt[st], 1);
-              if (o == ST_WARPS - 1) {
-                sh.mma_cnt[st] = 0;
-                if (st_wait(a_full(st), ph, abort_flag, err) && st_wait(b_full(st), ph, abort_flag, err)) {
-                  fence_after_sync();
-                  const uint32_t ah = base + (uint32_t)(st * ST_STAGE);
-                  const uint32_t al = ah + ST_A_PLANE, bh = ah + 2 * ST_A_PLANE, bl = bh + ST_B_PLANE;
-                  // the small cross products first, so that only the hi.hi steps round a full-size sum
-                  for (int kk = s_lo; kk <= s_hi; ++kk) {
-                    const uint32_t off = (uint32_t)kk * 32u;
-                    mma_f16(tmem, smem_desc(ah + off), smem_desc(bl + off), idesc,
-                            (c != c_lo || kk != s_lo) ? 1u : 0u);
-                    mma_f16(tmem, smem_desc(al + off), smem_desc(bh + off), idesc, 1u);
-                  }
-                  for (int kk = s_lo; kk <= s_hi; ++kk) {
-                    const uint32_t off = (uint32_t)kk * 32u;
-                    mma_f16(tmem, smem_desc(ah + off), smem_desc(bh + off), idesc, 1u);
-                  }
-                  mma_commit(s_empty(st));
-                  if (c == c_hi) mma_commit(d_full);
-                }
-                n_exec += (unsigned long long)ST_M * (ST_EPT * (s_hi - s_lo + 1)) * (nN / 2);
-              }
-            }
-            __syncwarp();
-            ++it;
-            ++n_items;
+            mbar_arrive_if(lead, d_empty(prv & 1u));
           }
         }
-        live = nlive;
-        if (!ok) break;
-        // the bin's Y: dot with the transmit phasors.  d_full is committed by the thread that
-        // issued the bin's last products; the item before it (another issuer, other stage)
-        // is complete when its stage is released (items on one stage complete in turn)
-        ok = __all_sync(0xffffffffu, st_wait(d_full, bn & 1u, abort_flag, err) &&
-                                         (n_items < 2 || st_wait(s_empty((int)(it & 1u)), ((it - 2) >> 1) & 1u,
-                                                                 abort_flag, err)));
-        if (!ok) break;
-        fence_after_sync();
-        float2 part = make_float2(0.0f, 0.0f);
-#pragma unroll
-        for (int c = 0; c < ST_CMAX; ++c) {
-          if (nlive & (1u << c)) {
-            const int col = 2 * ST_KC * c + 2 * ST_EPT * slot - 2 * (E0b - E0);
-            const int eb = E0 + ST_KC * c + ST_EPT * slot;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float yv[8];
-              tmem_ld8_nowait(tl + (uint32_t)(col + 8 * h), yv);
-              tmem_wait_ld();
-#pragma unroll
-              for (int kq = 0; kq < 4; ++kq) {
-                const int k2 = 4 * h + kq;
-                const float w = st_weight<WT>(d, eb + k2, emid, ta, tb, tLl, tLr, ic, d.wtx_par, ipt);
-                const float px = (k2 & 1) ? pr[c][k2 >> 1].y : pr[c][k2 >> 1].x;
-                const float py = (k2 & 1) ? pm[c][k2 >> 1].y : pm[c][k2 >> 1].x;
-                const float ar = w * px, ai = w * py;
-                const float yr = yv[2 * kq], yi = yv[2 * kq + 1];
-                part.x = fmaf(ar, yr, fmaf(-ai, yi, part.x));
-                part.y = fmaf(ar, yi, fmaf(ai, yr, part.y));
-              }
-            }
-          }
+        // n_k Y of the previous bin into the voxel, compensated
+        if (p_mask) {
+          const float yx = p_nrm * (sx.x + sx.y) - comp.x, nx = acc.x + yx;
+          comp.x = (nx - acc.x) - yx;
+          acc.x = nx;
+          const float yy = p_nrm * (sy.x + sy.y) - comp.y, ny = acc.y + yy;
+          comp.y = (ny - acc.y) - yy;
+          acc.y = ny;
         }
-        ++bn;
-        // n_k Y into the voxel, compensated
-        const float yx = nrm * part.x - comp.x, sx = acc.x + yx;
-        comp.x = (sx - acc.x) - yx;
-        acc.x = sx;
-        const float yy = nrm * part.y - comp.y, sy = acc.y + yy;
-        comp.y = (sy - acc.y) - yy;
-        acc.y = sy;
+        live = mask;
+        p_mask = mask;
+        p_rows = te.x;
+        p_nrm = __uint_as_float(te.y);
+        p_glo = g_lo;
+        p_wide = wide;
+        if (mask) ++nd;
       }
-    }
-    sh.red[slot][vb] = acc;
-    fence_before_sync();
-    __syncthreads();
-    fence_after_sync();
-    if (*abort_flag) break;
-    if (warp < 4 && vvalid) {
-      float sx = 0.0f, sy = 0.0f;
+      ns += (uint32_t)((nb + ST_TT - 1) / ST_TT);
+      {
+        const unsigned na = __reduce_add_sync(0xffffffffu, c_act), nm = __reduce_add_sync(0xffffffffu, c_emp);
+        if (lead) {
+          atomicAdd(&sh.n_active, (unsigned long long)na);
+          atomicAdd(&sh.n_empty, (unsigned long long)nm);
+        }
+      }
+      const size_t nvox = (size_t)d.nx * d.nz;
+      float2* out = d.split > 1 ? d.part + (size_t)part * nvox : image;
+      if (slot > 0) sh.red[slot - 1][vb] = acc;
+      p5_bar();
+      if (slot == 0 && valid) {
+        float2 o = acc;
 #pragma unroll
-      for (int s = 0; s < ST_WARPS / 4; ++s) {
-        sx += sh.red[s][vb].x;
-        sy += sh.red[s][vb].y;
+        for (int t = 0; t < 3; ++t) {
+          o.x += sh.red[t][vb].x;
+          o.y += sh.red[t][vb].y;
+        }
+        const float f = d.scale * inv_sigma;
+        out[vox] = make_float2(o.x * f, o.y * f);
       }
-      const float f = d.scale / sigma;
-      image[(size_t)ic * d.nz + jc] = make_float2(sx * f, sy * f);
+      if (d.split > 1) {
+        // the last of the tile's bin ranges to finish adds them up, in order
+        __threadfence();
+        p5_bar();
+        if (tid == 0)
+          sh.last = atomicAdd(&d.tile_cnt[(size_t)(d.wt_c0 / TILE_X) * ntz + tile], 1u) == (unsigned)(d.split - 1);
+        p5_bar();
+        if (sh.last && slot == 0 && valid) {
+          __threadfence();
+          float2 s = make_float2(0.0f, 0.0f);
+          for (int p = 0; p < d.split; ++p) {
+            const float2 v = __ldcg(d.part + (size_t)p * nvox + vox);
+            s.x += v.x;
+            s.y += v.y;
+          }
+          image[vox] = s;
+        }
+      }
+      __syncthreads();
     }
   }
-  atomicAdd(&d.counters[4], n_exec);
+  // after a timeout, give the copies and products in flight time to land before the tensor
+  // memory is freed (they take microseconds)
   if (tid == 0) {
     atomicAdd(&d.counters[0], sh.n_active);
     atomicAdd(&d.counters[1], sh.n_empty);
-    // after a timeout, give the copies and products in flight time to land before the
-    // tensor memory is freed (they take microseconds)
+    atomicAdd(&d.counters[4], sh.n_exec);
     if (*abort_flag) {
       const unsigned long long t0 = global_ns();
       while (global_ns() - t0 < 20000000ull) {
@@ -594,94 +674,113 @@ sa_tc_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ 
   __syncthreads();
   if (warp == 0) {
     fence_after_sync();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ST_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
 }
 
-typedef void (*st_kernel_t)(const CUtensorMap, const CUtensorMap, const SADev, const unsigned*, float2*, float*,
-                            float*, int, int);
-
-template <int WT>
-st_kernel_t st_pick_rx(int wr) {
-  switch (wr) {
-    case 0: return sa_tc_kernel<WT, 0>;
-    case 1: return sa_tc_kernel<WT, 1>;
-    case 2: return sa_tc_kernel<WT, 2>;
-    default: return sa_tc_kernel<WT, 4>;
-  }
+typedef void (*st_kernel_t)(const SADev, const uint4*, const unsigned*, float2*, float*, float*);
+st_kernel_t st_pick(const SADev& d) {
+  const bool lag = (d.ne + 7) / 8 <= ST_GMAX / 2, box = d.wtx_id == 0 && d.wrx_id == 0;
+  return lag ? (box ? sa_tc_kernel<true, true> : sa_tc_kernel<true, false>)
+             : (box ? sa_tc_kernel<false, true> : sa_tc_kernel<false, false>);
 }
-st_kernel_t st_pick(int wt, int wr) {
-  switch (wt) {
-    case 0: return st_pick_rx<0>(wr);
-    case 1: return st_pick_rx<1>(wr);
-    case 2: return st_pick_rx<2>(wr);
-    default: return st_pick_rx<4>(wr);
-  }
-}
+int st_smem(int G) { return st_sh_bytes() + 4 * ST_A + st_rho_bytes(G) + st_stages(G) * st_b_bytes(G); }
 
-// 3-D fp16 map over [bins][2 nep rows][2 nep columns], 64 x 64 boxes, 128-byte swizzle;
-// coordinates beyond the planes read as zero
-bool st_encode(CUtensorMap* m, const void* base, int nep, int K) {
-  EncodeTiled fn = encode_fn();
-  if (!fn) return false;
-  const cuuint64_t n = (cuuint64_t)(2 * nep);
-  const cuuint64_t dims[3] = {n, n, (cuuint64_t)K};
-  const cuuint64_t strides[2] = {n * 2, n * n * 2};
-  const cuuint32_t box[3] = {64, (cuuint32_t)ST_BOX_ROWS, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+int st_sms() {
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm > 0 ? nsm : 1;
 }
 
 }  // namespace
 
-bool sa_tc_supported(const SADev& d) { return d.ne >= 1 && d.ne <= ST_KC * ST_CMAX && d.last_bin_only == 0; }
+bool sa_tc_supported(const SADev& d) { return d.ne >= 1 && d.ne <= 8 * ST_GMAX && d.last_bin_only == 0; }
 
 size_t sa_tc_bytes(int ne, int K) {
-  const size_t nep = (size_t)((ne + 3) / 4 * 4);
-  return 2 * (size_t)K * (2 * nep) * (2 * nep) * sizeof(__half);
+  const size_t G = (size_t)((ne + 7) / 8);
+  return (size_t)K * G * G * 1024;
+}
+
+size_t sa_tc_scratch_bytes(const SADev& d) {
+  return (size_t)sa_tc_grid(d) * P5_M * 4 * ST_GMAX * sizeof(float4);
+}
+
+// Bin ranges per tile.  A tile is one block's work, so a frame of few tiles would leave SMs idle
+// in its last wave: its band is split into ranges of at least 64 bins (each pays the tile's
+// set-up) until there are about six items per SM.
+void sa_tc_pick_split(SADev& d) {
+  const int tiles = ((d.nx + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
+  int s = (6 * 152 + tiles - 1) / tiles;
+  s = std::max(1, std::min(s, d.K / 64));
+  d.split_bins = ((d.K + s - 1) / s + 31) / 32 * 32;
+  d.split = (d.K + d.split_bins - 1) / d.split_bins;
 }
 
 cudaError_t sa_tc_setup(SaTc& t, const SADev& d, void* planes, unsigned* maxbits, const float2* rot) {
-  t.nep = (d.ne + 3) / 4 * 4;
   t.planes = planes;
   t.maxbits = maxbits;
   t.rot = rot;
-  const size_t plane = (size_t)d.K * (2 * t.nep) * (2 * t.nep);
-  const __half* b = (const __half*)planes;
-  if (!st_encode(&t.tm[0], b, t.nep, d.K) || !st_encode(&t.tm[1], b + plane, t.nep, d.K))
-    return cudaErrorInvalidValue;
-  for (int wt : {0, 1, 2, 4})
-    for (int wr : {0, 1, 2, 4}) {
-      cudaError_t e = cudaFuncSetAttribute(st_pick(wt, wr), cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM);
-      if (e != cudaSuccess) return e;
-    }
-  return cudaSuccess;
+  // the compute warps' register share needs the full allocation at launch
+  cudaFuncAttributes a;
+  const void* fn = (const void*)st_pick(d);
+  cudaError_t e = cudaFuncGetAttributes(&a, fn);
+  if (e != cudaSuccess) return e;
+  if (a.numRegs != P5_REGS) return cudaErrorInvalidConfiguration;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM_MAX);
 }
 
 int sa_tc_grid(const SADev& d) {
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int tiles = ((d.nx + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
-  return std::max(1, std::min(tiles, nsm));
+  const int tiles = ((d.wt_nc + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z) * d.split;
+  return std::max(1, std::min(tiles, st_sms()));
 }
 
-cudaError_t launch_sa_tc(const SADev& d, const SaTc& t, int grid, float2* image, float* wtx, float* wrx,
-                         cudaStream_t s) {
-  const int ntx = (d.nx + TILE_X - 1) / TILE_X, ntz = (d.nz + TILE_Z - 1) / TILE_Z;
-  cudaError_t e = cudaMemsetAsync(d.counters + 3, 0, sizeof(unsigned long long), s);
+// one window table per side for the columns wt_c0 .. wt_c0 + wt_nc - 1
+cudaError_t launch_sa_tc_window(const SADev& d, cudaStream_t s) {
+  PWDev w{};
+  w.ne = d.ne;
+  w.ne_pad = d.ne_pad;
+  w.wt_c0 = d.wt_c0;
+  w.wt_nc = d.wt_nc;
+  w.col_m = d.col_m;
+  w.col_emid = d.col_emid;
+  w.el_m = d.el_m;
+  w.el_lb = d.el_lb;
+  w.el_ub = d.el_ub;
+  w.pitch_f = d.pitch_f;
+  for (int i = 0; i < (d.w_tab[0] == d.w_tab[1] ? 1 : 2); ++i) {
+    w.window_id = i ? d.wrx_id : d.wtx_id;
+    w.window_par = i ? d.wrx_par : d.wtx_par;
+    const cudaError_t e = launch_pw_tc_window(w, const_cast<float*>(d.w_tab[i]), const_cast<float*>(d.w_sum[i]), s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_sa_tc(const SADev& d0, const SaTc& t, float2* image, float* wtx, float* wrx, cudaStream_t s) {
+  cudaError_t e = launch_absmax((const float*)d0.X, (size_t)d0.ne * d0.ne * d0.K * 2, t.maxbits, s);
   if (e != cudaSuccess) return e;
-  if ((e = launch_absmax((const float*)d.X, (size_t)d.ne * d.ne * d.K * 2, t.maxbits, s)) != cudaSuccess) return e;
-  const size_t plane = (size_t)d.K * (2 * t.nep) * (2 * t.nep) / 2;   // half2 per plane
-  __half2* bhi = (__half2*)t.planes;
-  const dim3 pg(t.nep, (t.nep + 31) / 32, (d.K + 31) / 32);
-  sa_tc_prep_kernel<<<pg, 256, 0, s>>>(d.X, d.ne, t.nep, d.K, t.rot, t.maxbits, bhi, bhi + plane);
+  const int G = (d0.ne + 7) / 8;
+  const dim3 pg(2 * G, (G + 3) / 4, (d0.K + 7) / 8);
+  sa_tc_prep_kernel<<<pg, 256, 0, s>>>(d0.X, d0.ne, G, d0.K, t.rot, t.maxbits, (uint4*)t.planes);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  st_pick(d.wtx_id, d.wrx_id)<<<grid, ST_THREADS, ST_SMEM, s>>>(t.tm[0], t.tm[1], d, t.maxbits, image, wtx, wrx,
-                                                                 ntx, ntz);
-  return cudaGetLastError();
+  SADev d = d0;
+  if (d.split > 1) {
+    const size_t tiles = (size_t)((d.nx + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
+    if ((e = cudaMemsetAsync(d.tile_cnt, 0, tiles * sizeof(unsigned), s)) != cudaSuccess) return e;
+  }
+  for (int c0 = 0; c0 < d0.nx; c0 += d0.wt_nc) {
+    d.wt_c0 = c0;
+    d.wt_nc = std::min(d0.wt_nc, d0.nx - c0);
+    // window tables that do not hold all columns are refilled for each slab of them
+    if (d0.wt_nc < d0.nx && (e = launch_sa_tc_window(d, s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(d.counters + 3, 0, sizeof(unsigned long long), s)) != cudaSuccess) return e;
+    st_pick(d)<<<sa_tc_grid(d), P5_THREADS, st_smem(G), s>>>(d, (const uint4*)t.planes, t.maxbits, image, wtx, wrx);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace fnum
