@@ -449,15 +449,14 @@ struct fnum_plan {
   // sharpness-loss gradients (fnum_pw_sharpness_grad), allocated on first use
   float2* adj_img = nullptr;
   float2* adj_G = nullptr;     // cotangent dL/dI* of the sharpness loss
-  float* adj_invw = nullptr;
   float2* adj_D = nullptr;     // Draw of the derivative forward (dI/dc = -(2 pi i / c) Draw)
   float2* adj_gX = nullptr;
   double* adj_sums = nullptr;
   double* adj_acc = nullptr;   // FP64 sums of the voxel slices, 2 per spectrum entry
   float4* adj_rx = nullptr;    // receive delays and steps of the adjoint (PWDev::rx_tab)
   bool adj_rx_tried = false;
-  unsigned* adj_gmax = nullptr;  // fp16 scale inputs of the adjoint: max |G|, max 1/W
-  bool adj_invw_ready = false;
+  unsigned* adj_gmax = nullptr;  // fp16 scale inputs of the adjoint: max |G|, max n_k
+  bool adj_nmax_ready = false;
   // band DFT on the tensor cores: fp16 hi/lo operand planes, per-line scales, TMA maps
   fnum::DftTc dft{};
   // synthetic aperture on the tensor cores: operand planes, TMA maps, scale word and
@@ -1924,8 +1923,8 @@ int fnum_pw_plan_set_sound_speed(fnum_plan* plan, double c_0) {
 
 namespace fnum {
 
-// gradient buffers of a compounded plane-wave plan, allocated on first use; the 1/W
-// table of the frozen apertures is built once
+// gradient buffers of a compounded plane-wave plan, allocated on first use; the largest n_k of
+// the frozen apertures is taken once
 int adjoint_buffers(fnum_plan* plan, cudaStream_t st) {
   const fnum::PWDev& D = plan->pw;
   const long long nvox = (long long)D.nx * D.nz;
@@ -1933,7 +1932,7 @@ int adjoint_buffers(fnum_plan* plan, cudaStream_t st) {
   int s = FNUM_OK;
   if (!plan->adj_img) {
     if ((s = plan->alloc(&plan->adj_img, (size_t)nvox)) || (s = plan->alloc(&plan->adj_G, (size_t)nvox)) ||
-        (s = plan->alloc(&plan->adj_invw, (size_t)nvox * D.K)) || (s = plan->alloc(&plan->adj_D, (size_t)nvox)) ||
+        (s = plan->alloc(&plan->adj_D, (size_t)nvox)) ||
         (s = plan->alloc(&plan->adj_gX, nspec)) || (s = plan->alloc(&plan->adj_sums, 4)) ||
         (s = plan->alloc(&plan->adj_acc, 2 * nspec)) || (s = plan->alloc(&plan->adj_gmax, 2)))
       return s;
@@ -1944,10 +1943,9 @@ int adjoint_buffers(fnum_plan* plan, cudaStream_t st) {
     plan->adj_rx_tried = true;
     if (plan->alloc(&plan->adj_rx, (size_t)nvox * D.ne) == FNUM_OK) plan->pw.rx_tab = plan->adj_rx;
   }
-  if (!plan->adj_invw_ready) {
-    FNUM_CUDA(fnum::launch_pw_invw(D, plan->adj_invw, st));
-    FNUM_CUDA(fnum::launch_absmax(plan->adj_invw, (size_t)nvox * D.K, plan->adj_gmax + 1, st));
-    plan->adj_invw_ready = true;
+  if (!plan->adj_nmax_ready) {
+    FNUM_CUDA(fnum::launch_pw_nmax(D, plan->adj_gmax + 1, st));
+    plan->adj_nmax_ready = true;
   }
   return FNUM_OK;
 }
@@ -1963,15 +1961,14 @@ int adjoint_core(fnum_plan* plan, const float2* G, float2* gX, double* dloss_dc,
     if (!have_D) FNUM_CUDA(fnum::launch_pw_mma_deriv(D, plan->max_grid, plan->adj_img, plan->adj_D, st));
     FNUM_CUDA(fnum::launch_pw_dc_reduce(G, plan->adj_D, nvox, 4.0 * M_PI / plan->c, plan->adj_sums + 2, st));
   }
-  if (gX) FNUM_CUDA(fnum::launch_pw_adjoint(D, G, plan->adj_invw, plan->adj_gmax, gX, plan->adj_acc, st));
-  if (dloss_dc) {
-    double g = 0.0;
-    FNUM_CUDA(cudaMemcpyAsync(&g, plan->adj_sums + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
-    FNUM_CUDA(cudaStreamSynchronize(st));
-    *dloss_dc = g;
-  } else {
-    FNUM_CUDA(cudaStreamSynchronize(st));
-  }
+  if (gX) FNUM_CUDA(fnum::launch_pw_adjoint(D, G, plan->adj_gmax, gX, plan->adj_acc, st));
+  double g = 0.0;
+  unsigned long long err = 0;
+  if (dloss_dc) FNUM_CUDA(cudaMemcpyAsync(&g, plan->adj_sums + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
+  FNUM_CUDA(cudaMemcpyAsync(&err, plan->counters + 2, sizeof(err), cudaMemcpyDeviceToHost, st));
+  FNUM_CUDA(cudaStreamSynchronize(st));
+  if (err & fnum::ERR_TC_TIMEOUT) return FNUM_ERR_INTERNAL;
+  if (dloss_dc) *dloss_dc = g;
   return FNUM_OK;
 }
 

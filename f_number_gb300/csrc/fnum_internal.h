@@ -248,15 +248,16 @@ cudaError_t launch_pw_m(const PWDev& d, int compound, float2* image, float* weig
 cudaError_t launch_sa_fused(const SADev& d, int grid, float2* image, float* wtx, float* wrx, cudaStream_t s);
 cudaError_t launch_sa_plain(const SADev& d, float2* image, float* wtx, float* wrx, cudaStream_t s);
 // sharpness-loss gradients of a compounded plane-wave plan (fnum_pw_sharpness_grad)
-cudaError_t launch_pw_invw(const PWDev& d, float* invw, cudaStream_t s);
+// largest n_k of the frame (float bits) into *out
+cudaError_t launch_pw_nmax(const PWDev& d, unsigned* out, cudaStream_t s);
 cudaError_t launch_pw_sharp_sums(const float2* img, long long n, double* sums, cudaStream_t s);
 // G = dL/dI* of the sharpness loss from the image and its sums (gs2 = 1/S2^2, gs4 = S4/S2^3)
 cudaError_t launch_pw_sharp_cotangent(const float2* img, long long n, float gs2, float gs4, float2* G, cudaStream_t s);
 // adjoint of the compounded beamformer for a cotangent G = dL/dI* [nx][nz] on the tensor
 // cores: gX = dL/dX*; acc: 2 doubles per spectrum entry
-// gmax: two device words, [1] = max 1/W (launch_absmax over the 1/W table, once), [0] set here
-cudaError_t launch_pw_adjoint(const PWDev& d, const float2* cot, const float* invw, unsigned* gmax, float2* gX,
-                              double* acc, cudaStream_t s);
+// gmax: two device words, [1] = max n_k (launch_pw_nmax, once), [0] set here
+cudaError_t launch_pw_adjoint(const PWDev& d, const float2* cot, unsigned* gmax, float2* gX, double* acc,
+                              cudaStream_t s);
 // float bits of max |x_i| of n floats into *out
 cudaError_t launch_absmax(const float* x, size_t n, unsigned* out, cudaStream_t s);
 // dL/dc = coef sum_v Im(conj(G_v) D_v) into *out (FP64)

@@ -2310,9 +2310,9 @@ namespace fnum {
 // No counterpart in the reference.
 // ---------------------------------------------------------------------------
 
-// 1/W (or 1, or 0 for an empty aperture) per voxel and band bin: [voxel][K]
+// largest 1/W (or 1, or 0 for empty apertures) over voxels and band bins, as float bits
 template <int WIN>
-__global__ void __launch_bounds__(NTHREADS) pw_invw_kernel(const PWDev d, float* __restrict__ invw) {
+__global__ void __launch_bounds__(NTHREADS) pw_nmax_kernel(const PWDev d, unsigned* __restrict__ out) {
   const long long v = (long long)blockIdx.x * NTHREADS + threadIdx.x;
   if (v >= (long long)d.nx * d.nz) return;
   const int i = (int)(v / d.nz), j = (int)(v - (long long)i * d.nz);
@@ -2320,7 +2320,7 @@ __global__ void __launch_bounds__(NTHREADS) pw_invw_kernel(const PWDev d, float*
   const int emid = d.col_emid[i];
   const float inv_par = (d.window_par > 0.0f) ? 1.0f / d.window_par : 0.0f;
   int prev = -1;
-  float iw = 0.0f;
+  float top = 0.0f;
   for (int kk = 0; kk < d.K; ++kk) {
     int ilb, iub;
     aperture(xp, zp, d.g[kk], d.ne, ilb, iub);
@@ -2329,11 +2329,11 @@ __global__ void __launch_bounds__(NTHREADS) pw_invw_kernel(const PWDev d, float*
       const float Ll = half_left(d.el_lb, xm, ilb, d.ne), Lr = half_right(d.el_ub, xm, iub);
       const float W = aperture_sum_closed<WIN>(d, inv_par, xm, emid, ilb, iub, (Ll > 0.0f) ? 1.0f / Ll : 0.0f,
                                                (Lr > 0.0f) ? 1.0f / Lr : 0.0f);
-      iw = (W > 0.0f) ? (d.norm ? 1.0f / W : 1.0f) : 0.0f;
+      top = fmaxf(top, (W > 0.0f) ? (d.norm ? 1.0f / W : 1.0f) : 0.0f);
       prev = code;
     }
-    invw[(size_t)v * d.K + kk] = iw;
   }
+  atomicMax(out, __float_as_uint(top));
 }
 
 // S2, S4 of an image (double accumulation)
@@ -2386,14 +2386,16 @@ __global__ void __launch_bounds__(256) pw_dc_reduce_kernel(const float2* __restr
   }
 }
 
-cudaError_t launch_pw_invw(const PWDev& d, float* invw, cudaStream_t s) {
+cudaError_t launch_pw_nmax(const PWDev& d, unsigned* out, cudaStream_t s) {
   const long long nv = (long long)d.nx * d.nz;
+  const cudaError_t e = cudaMemsetAsync(out, 0, sizeof(unsigned), s);
+  if (e != cudaSuccess) return e;
   const int grid = (int)((nv + NTHREADS - 1) / NTHREADS);
   switch (d.window_id) {
-    case 0: pw_invw_kernel<0><<<grid, NTHREADS, 0, s>>>(d, invw); break;
-    case 1: pw_invw_kernel<1><<<grid, NTHREADS, 0, s>>>(d, invw); break;
-    case 2: pw_invw_kernel<2><<<grid, NTHREADS, 0, s>>>(d, invw); break;
-    default: pw_invw_kernel<4><<<grid, NTHREADS, 0, s>>>(d, invw); break;
+    case 0: pw_nmax_kernel<0><<<grid, NTHREADS, 0, s>>>(d, out); break;
+    case 1: pw_nmax_kernel<1><<<grid, NTHREADS, 0, s>>>(d, out); break;
+    case 2: pw_nmax_kernel<2><<<grid, NTHREADS, 0, s>>>(d, out); break;
+    default: pw_nmax_kernel<4><<<grid, NTHREADS, 0, s>>>(d, out); break;
   }
   return cudaGetLastError();
 }
@@ -2420,16 +2422,6 @@ cudaError_t launch_pw_sharp_cotangent(const float2* img, long long n, float gs2,
   return cudaGetLastError();
 }
 
-// fp16 scale of Q = conj(t^k) G / W: the power of two that brings max|G| max(1/W), a bound
-// of |Q|, below 2^14 (gmax: float bits of max |G component| and of max 1/W)
-__device__ __forceinline__ float adj_scale(const unsigned* gmax) {
-  const float m = __uint_as_float(gmax[0]) * __uint_as_float(gmax[1]);
-  if (!(m > 0.0f) || !(m < 3.0e38f)) return 1.0f;
-  int ex;
-  frexpf(m, &ex);
-  return ldexpf(1.0f, min(max(14 - ex, -126), 126));
-}
-
 // largest |x| of n floats (float bits, >= 0 floats order as integers) into *out
 __global__ void __launch_bounds__(256) absmax_f32_kernel(const float* __restrict__ x, size_t n, unsigned* out) {
   float m = 0.0f;
@@ -2437,308 +2429,6 @@ __global__ void __launch_bounds__(256) absmax_f32_kernel(const float* __restrict
     m = fmaxf(m, fabsf(x[i]));
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
-}
-
-// FP64 sums {Xr, Xi} per (element, bin, angle) -> dL/dX* (scaled by 2/N, the fp16 scale undone)
-__global__ void __launch_bounds__(256) pw_adjoint_finish_kernel(const double* __restrict__ acc, size_t n, double scale,
-                                                                const unsigned* __restrict__ gmax,
-                                                                float2* __restrict__ gX) {
-  const double sc = scale / (double)adj_scale(gmax);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double* a = acc + 2 * i;
-    gX[i] = make_float2((float)(sc * a[0]), (float)(sc * a[1]));
-  }
-}
-
-// ---------------------------------------------------------------------------
-// The adjoint on the tensor cores: per band bin k,
-//   gX_k(e, a) = s sum_v conj(R_k(v, e)) Q_k(v, a),  R_k = b r^k,  Q_k = conj(t_va^k) G_v / W_vk,
-// an [elements x voxels] . [voxels x angles] product reduced over the voxels (the
-// forward's product transposed).  Block: 8 warps, warp w owns elements 16w..16w+15 of
-// the block's element pass (mma rows); the voxels are the mma k dimension (8 complex per
-// k-step, real form: columns 0..7 Re, 8..15 Im of conj(R)) and the angles the n dimension
-// (3 tiles of 4).  A block takes one chunk of ADJ_TB bins and one slice of voxels; per
-// group of 8 voxels it stages the aperture data and the B fragments of Q (fp16 hi and lo,
-// scaled by a power of two) in shared memory, then each warp forms conj(R) for its 16
-// elements x 8 voxels -- the receive phasor anchored exactly at the chunk's top bin and
-// stepped down by r -- and accumulates the chunk's bins in registers (ADJ_TB x 12 floats).
-// At the end of the slice the sums are added to FP64 accumulators.
-constexpr int ADJ_TB = 6;           // bins per chunk (register accumulators per bin)
-constexpr int ADJ_TC_SLICE = 8192;  // voxels per block
-constexpr int ADJ_TC_WARPS = 8;
-
-// e^{j 2 pi k u} with the exact reduction of cis_ku and the hardware sine and cosine of the
-// reduced angle (absolute error below 4e-7): the adjoint's anchors
-__device__ __forceinline__ float2 cis_ku_fast(int k, dfl u) {
-  const float kf = (float)k;
-  dfl p = two_prod(kf, u.x);
-  const float n = rintf(p.x);
-  const float rh = p.x - n;
-  const float rl = fmaf(kf, u.y, p.y);
-  const float r = rh + rl;
-  float sn, cs;
-  __sincosf(6.28318530717958647692f * r, &sn, &cs);
-  return make_float2(cs, sn);
-}
-
-// the adjoint's receive table: u_rx in double-float and the step e^{2 pi i u_rx} of every
-// (voxel, element) pair, formed as pw_adjoint_tc_kernel forms them without the table
-__global__ void __launch_bounds__(256) pw_rx_table_kernel(const PWDev d) {
-  const size_t n = (size_t)d.nx * d.nz * d.ne;
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
-    const size_t v = idx / d.ne;
-    const int e = (int)(idx - v * d.ne);
-    const int i = (int)(v / d.nz), j = (int)(v - (size_t)i * d.nz);
-    const dfl urx = df_sqrt(df_add(df_sqr(df_sub(d.el_u[e], d.col_u[i])), d.row_u2[j]));
-    const float2 st = cis_ku_fast(1, urx);
-    d.rx_tab[idx] = make_float4(urx.x, urx.y, st.x, st.y);
-  }
-}
-
-template <int WIN>
-__global__ void __launch_bounds__(ADJ_TC_WARPS * 32, 2)
-pw_adjoint_tc_kernel(const PWDev d, const float2* __restrict__ cot, const float* __restrict__ invw,
-                     const unsigned* __restrict__ gmax, double* __restrict__ acc) {
-  __shared__ float2 sQ[ADJ_TB][8][TC_NA];        // Q_k(v, a) sigma
-  __shared__ uint4 sB[ADJ_TB][3][32];            // B fragments {b0 hi, b1 hi, b0 lo, b1 lo}
-  __shared__ float2 sAp[ADJ_TB][8];              // {1/L_left, 1/L_right} per bin, voxel (1e30: no side)
-  __shared__ int sVox[8][3];                     // column, row, first element right of x
-  __shared__ int2 sRng[ADJ_TB][8];               // aperture element range {ilb, iub} per bin, voxel
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, q = lane & 3;
-  const int kc_lo = d.k_lb + blockIdx.x * ADJ_TB, kc_hi = min(kc_lo + ADJ_TB, d.k_ub + 1) - 1;
-  const int nb = kc_hi - kc_lo + 1;
-  const long long nvox = (long long)d.nx * d.nz;
-  const long long v_begin = (long long)blockIdx.y * ADJ_TC_SLICE;
-  const long long v_end = min(nvox, v_begin + ADJ_TC_SLICE);
-  const int e_pass = blockIdx.z * (ADJ_TC_WARPS * 16);
-  const int eA = e_pass + 16 * warp + g, eB = eA + 8;   // the thread's elements (mma rows g, g + 8)
-  const dfl cmA = d.el_m[min(eA, d.ne - 1)], cmB = d.el_m[min(eB, d.ne - 1)];
-  const dfl cuA = d.el_u[min(eA, d.ne - 1)], cuB = d.el_u[min(eB, d.ne - 1)];
-  const float inv_par = (d.window_par > 0.0f) ? 1.0f / d.window_par : 0.0f;
-  const float sigma = adj_scale(gmax);
-  float C[ADJ_TB][3][4];
-#pragma unroll
-  for (int b = 0; b < ADJ_TB; ++b)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) C[b][j][0] = C[b][j][1] = C[b][j][2] = C[b][j][3] = 0.0f;
-
-  for (long long v0 = v_begin; v0 < v_end; v0 += 8) {
-    const int nv = (int)min(8ll, v_end - v0);
-    __syncthreads();   // the previous group's tables are consumed
-    if (tid < 8) {
-      const long long v = v0 + min(tid, nv - 1);
-      const int i = (int)(v / d.nz), j = (int)(v - (long long)i * d.nz);
-      sVox[tid][0] = i;
-      sVox[tid][1] = j;
-      sVox[tid][2] = d.col_emid[i];
-    }
-    __syncthreads();
-    // Q (96 threads: voxel x angle) and the aperture data (ADJ_TB x 8 threads)
-    if (tid < 8 * TC_NA) {
-      const int vv = tid / TC_NA, a = tid - vv * TC_NA;
-      float2 base = make_float2(0.0f, 0.0f), t = make_float2(1.0f, 0.0f);
-      if (vv < nv && a < d.na) {
-        const int i = sVox[vv][0], j = sVox[vv][1];
-        const dfl ut = df_add(d.tx_ax[(size_t)a * d.nx + i], d.tx_az[(size_t)a * d.nz + j]);
-        const float2 c = cis_ku_fast(kc_hi, ut);
-        const float2 G = cot[v0 + vv];
-        t = cis_ku_fast(1, ut);
-        // conj(t^k) G sigma at the top bin; going down, conj(t^(k-1)) = conj(t^k) t
-        base = make_float2(sigma * (G.x * c.x + G.y * c.y), sigma * (G.y * c.x - G.x * c.y));
-      }
-#pragma unroll
-      for (int b = 0; b < ADJ_TB; ++b) {
-        float2 qv = make_float2(0.0f, 0.0f);
-        if (vv < nv && a < d.na && b < nb) {
-          const float iw = invw[(size_t)(v0 + vv) * d.K + (kc_hi - b - d.k_lb)];
-          qv = make_float2(base.x * iw, base.y * iw);
-        }
-        sQ[b][vv][a] = qv;
-        base = cmul(base, t);
-      }
-    } else if (tid >= 128 && tid < 128 + ADJ_TB * 8) {
-      const int b = (tid - 128) >> 3, vv = (tid - 128) & 7;
-      float il = 1.0e30f, ir = 1.0e30f;
-      int2 rng = make_int2(d.ne, -1);
-      if (vv < nv && b < nb) {
-        const int i = sVox[vv][0], j = sVox[vv][1];
-        const dfl xm = d.col_m[i];
-        int ilb, iub;
-        aperture(d.col_p[i], d.row_p[j], d.g[kc_hi - b - d.k_lb], d.ne, ilb, iub);
-        rng = make_int2(ilb, iub);
-        if (ilb < d.ne) {
-          const dfl l = d.el_lb[ilb];
-          const float L = (xm.x - l.x) + (xm.y - l.y);
-          if (L > 0.0f) il = __fdividef(1.0f, L);
-        }
-        if (iub >= 0) {
-          const dfl u = d.el_ub[iub];
-          const float L = (u.x - xm.x) + (u.y - xm.y);
-          if (L > 0.0f) ir = __fdividef(1.0f, L);
-        }
-      }
-      sAp[b][vv] = make_float2(il, ir);
-      sRng[b][vv] = rng;
-    }
-    __syncthreads();
-    // B fragments: lane (gg, qq) of n-tile j holds rows 2qq, 2qq+1 (voxels, Re block) and
-    // 2qq+8, 2qq+9 (second block) of column gg = angle 4j + gg/2, part gg%2
-    for (int f = tid; f < ADJ_TB * 3 * 32; f += ADJ_TC_WARPS * 32) {
-      const int b = f / 96, j = (f / 32) % 3, ln = f & 31;
-      const int gg = ln >> 2, qq = ln & 3, a = 4 * j + (gg >> 1), part = gg & 1;
-      float r0[2], r1[2];
-#pragma unroll
-      for (int t2 = 0; t2 < 2; ++t2) {
-        const float2 qv = sQ[b][2 * qq + t2][a];
-        r0[t2] = part ? qv.y : qv.x;     // rows 0..7:  Re Q (column re) / Im Q (column im)
-        r1[t2] = part ? qv.x : -qv.y;    // rows 8..15: -Im Q / Re Q
-      }
-      uint4 o;
-      tc_split(r0[0], r0[1], o.x, o.z);
-      tc_split(r1[0], r1[1], o.y, o.w);
-      sB[b][j][ln] = o;
-    }
-    __syncthreads();
-    // The bins in which one of the warp's 16 elements lies in the aperture range of one
-    // of the 8 voxels: elements outside [ilb, iub] have window argument u >= 1 (weight
-    // 0), so the other bins add nothing and are skipped, and with them the whole group
-    // when none is left.  Lane p checks (bin p / 8, voxel p % 8) and p + 32.
-    unsigned act = 0;
-    {
-      const int w_lo = e_pass + 16 * warp, w_hi = min(w_lo + 15, d.ne - 1);
-      bool h0 = false, h1 = false;
-      if (lane < ADJ_TB * 8) {
-        const int2 r = sRng[lane >> 3][lane & 7];
-        h0 = max(r.x, w_lo) <= min(r.y, w_hi);
-      }
-      if (lane + 32 < ADJ_TB * 8) {
-        const int2 r = sRng[(lane + 32) >> 3][lane & 7];
-        h1 = max(r.x, w_lo) <= min(r.y, w_hi);
-      }
-      const unsigned m0 = __ballot_sync(0xffffffffu, h0), m1 = __ballot_sync(0xffffffffu, h1);
-#pragma unroll
-      for (int b = 0; b < ADJ_TB; ++b) {
-        const unsigned byte = (b < 4) ? (m0 >> (8 * b)) : (m1 >> (8 * (b - 4)));
-        if (byte & 0xffu) act |= 1u << b;
-      }
-    }
-    if (act == 0) continue;
-    // conj(R) of elements (eA, eB) x voxels (2q, 2q+1)
-    float2 P[2][2], st[2][2];   // [element][voxel]: conj(r^k) and the step r
-    float dl[2][2], dr[2][2];   // distances to the voxel by aperture side
-#pragma unroll
-    for (int t2 = 0; t2 < 2; ++t2) {
-      const int vv = 2 * q + t2;
-      const int i = sVox[vv][0], j = sVox[vv][1];
-      const dfl xm = d.col_m[i];
-      const int emid = sVox[vv][2];
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const dfl cm = m ? cmB : cmA;
-        const int e = m ? eB : eA;
-        dfl urx;
-        if (d.rx_tab) {
-          const float4 rx = d.rx_tab[(size_t)(v0 + min(vv, nv - 1)) * d.ne + min(e, d.ne - 1)];
-          urx = make_float2(rx.x, rx.y);
-          st[m][t2] = make_float2(rx.z, rx.w);
-        } else {
-          const dfl cu = m ? cuB : cuA;
-          urx = df_sqrt(df_add(df_sqr(df_sub(cu, d.col_u[i])), d.row_u2[j]));
-          st[m][t2] = cis_ku_fast(1, urx);
-        }
-        const float2 c = cis_ku_fast(kc_hi, urx);
-        P[m][t2] = make_float2(c.x, -c.y);
-        const float dx = fabsf((cm.x - xm.x) + (cm.y - xm.y));
-        const bool ok = (vv < nv) && (e < d.ne);
-        const bool left = e < emid;
-        dl[m][t2] = ok ? (left ? dx : 0.0f) : 1.0e30f;   // an empty slot lies outside every aperture
-        dr[m][t2] = ok ? (left ? 0.0f : dx) : 0.0f;
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < ADJ_TB; ++b) {
-      if (b < nb && !((act >> b) & 1u)) {
-#pragma unroll
-        for (int t2 = 0; t2 < 2; ++t2)
-#pragma unroll
-          for (int m = 0; m < 2; ++m) P[m][t2] = cmul(P[m][t2], st[m][t2]);
-      } else if (b < nb) {
-        float rr[2][2], ri[2][2];
-#pragma unroll
-        for (int t2 = 0; t2 < 2; ++t2) {
-          const float2 ap = sAp[b][2 * q + t2];
-#pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            const float u = fmaf(dl[m][t2], ap.x, dr[m][t2] * ap.y);
-            const float w = (u < 1.0f) ? win_t<WIN>(d.window_par, inv_par, u) : 0.0f;
-            const float2 pc = P[m][t2];
-            rr[m][t2] = w * pc.x;          // Re conj(R)
-            ri[m][t2] = w * pc.y;          // Im conj(R)
-            P[m][t2] = cmul(pc, st[m][t2]);
-          }
-        }
-        unsigned ah[4], al[4];
-        tc_split(rr[0][0], rr[0][1], ah[0], al[0]);   // row g:     columns 2q, 2q+1
-        tc_split(rr[1][0], rr[1][1], ah[1], al[1]);   // row g + 8
-        tc_split(ri[0][0], ri[0][1], ah[2], al[2]);   // row g:     columns 2q+8, 2q+9
-        tc_split(ri[1][0], ri[1][1], ah[3], al[3]);   // row g + 8
-        uint4 bf[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) bf[j] = sB[b][j][lane];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) tc_mma(C[b][j], ah, bf[j].x, bf[j].y);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) tc_mma(C[b][j], ah, bf[j].z, bf[j].w);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) tc_mma(C[b][j], al, bf[j].x, bf[j].y);
-      }
-    }
-  }
-  // C[b][j]: rows g, g+8 (elements eA, eB), columns 2q, 2q+1 (angle 4j + q: re, im)
-#pragma unroll
-  for (int b = 0; b < ADJ_TB; ++b) {
-    if (b >= nb) continue;
-    const int kk = kc_hi - b - d.k_lb;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int a = 4 * j + q;
-      if (a >= d.na) continue;
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const int e = m ? eB : eA;
-        if (e >= d.ne) continue;
-        double* o = acc + 2 * (((size_t)e * d.K + kk) * d.na + a);
-        atomicAdd(o, (double)C[b][j][2 * m]);
-        atomicAdd(o + 1, (double)C[b][j][2 * m + 1]);
-      }
-    }
-  }
-}
-
-cudaError_t launch_pw_adjoint(const PWDev& d, const float2* cot, const float* invw, unsigned* gmax, float2* gX,
-                              double* acc, cudaStream_t s) {
-  const size_t n = (size_t)d.ne * d.K * d.na;
-  const long long nvox = (long long)d.nx * d.nz;
-  // gmax[1] (max 1/W) is set once with the 1/W table; max |G| per call
-  cudaError_t e = cudaMemsetAsync(acc, 0, 2 * n * sizeof(double), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(gmax, 0, sizeof(unsigned), s);
-  if (e != cudaSuccess) return e;
-  absmax_f32_kernel<<<608, 256, 0, s>>>(reinterpret_cast<const float*>(cot), 2 * (size_t)nvox, gmax);
-  if (d.rx_tab) pw_rx_table_kernel<<<1216, 256, 0, s>>>(d);
-  const dim3 grid((d.K + ADJ_TB - 1) / ADJ_TB, (unsigned)((nvox + ADJ_TC_SLICE - 1) / ADJ_TC_SLICE),
-                  (d.ne + ADJ_TC_WARPS * 16 - 1) / (ADJ_TC_WARPS * 16));
-  const int nt = ADJ_TC_WARPS * 32;
-  switch (d.window_id) {
-    case 0: pw_adjoint_tc_kernel<0><<<grid, nt, 0, s>>>(d, cot, invw, gmax, acc); break;
-    case 1: pw_adjoint_tc_kernel<1><<<grid, nt, 0, s>>>(d, cot, invw, gmax, acc); break;
-    case 2: pw_adjoint_tc_kernel<2><<<grid, nt, 0, s>>>(d, cot, invw, gmax, acc); break;
-    default: pw_adjoint_tc_kernel<4><<<grid, nt, 0, s>>>(d, cot, invw, gmax, acc); break;
-  }
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  pw_adjoint_finish_kernel<<<608, 256, 0, s>>>(acc, n, (double)d.scale, gmax, gX);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_absmax(const float* x, size_t n, unsigned* out, cudaStream_t s) {
