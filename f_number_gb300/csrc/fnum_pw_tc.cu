@@ -82,9 +82,13 @@ struct P5Shared {
   uint64_t bars[2 * 4 + 2 * 2 + 4 + 2 * P5_NT];
 };
 
+// Element groups a pass holds at most: all of a short array, else 8, which leave half of the
+// block's shared memory to the L1 cache that the window loads want (128 elements, 11 angles,
+// 512 x 512: 15.9 ms, with 12 groups 16.2; 96 elements, 5 angles: 1.92 and 1.79 ms).  A frame's
+// own, so that it sums in the same order in a batch.
+__host__ __device__ inline int p5_groups(const PWDev& d) { return d.ne <= 96 && d.na <= 16 ? 12 : 8; }
 // groups per element pass: the tile's groups in as few passes as hold them, of equal width
-template <int GP>
-__device__ __forceinline__ int p5_pass(int E_lo, int E_hi) {
+__device__ __forceinline__ int p5_pass(int GP, int E_lo, int E_hi) {
   if (E_lo > E_hi) return GP;
   const int n = (E_hi >> 3) - (E_lo >> 3) + 1, passes = (n + GP - 1) / GP;
   return (n + passes - 1) / passes;
@@ -190,7 +194,7 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
       __syncthreads();
       const unsigned un = p5_uni(p5_join(sh.un));
       const int E_lo = (int)(un & 0xffffu), E_hi = un == 0xffffffffu ? -1 : 0xffff - (int)(un >> 16);
-      const int gp = p5_pass<GP>(E_lo, E_hi);
+      const int gp = p5_pass(BATCH ? min(p5_groups(d), GP) : GP, E_lo, E_hi);
       const int role = warp - P5_CW;       // 0, 1: products of the first, second bin of a pair; 2: copies
       if (lane == 0 && role < 3) {
         const int n_grp = d.ne_pad >> 3;                      // element groups of 8 in the spectra
@@ -312,7 +316,7 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
       __syncthreads();
       const unsigned un = p5_uni(p5_join(sh.un));
       const int E_lo = (int)(un & 0xffffu), E_hi = un == 0xffffffffu ? -1 : 0xffff - (int)(un >> 16);
-      const int gp = p5_pass<GP>(E_lo, E_hi);
+      const int gp = p5_pass(BATCH ? min(p5_groups(d), GP) : GP, E_lo, E_hi);
       const float inv_sigma = 1.0f / tc_scale(*d.tc_max);
       const int n_grp = d.ne_pad >> 3;                      // element groups of 8 in the spectra
       const int tb = (d.tc_tb > 0 && d.tc_tb < 32) ? d.tc_tb : 32;   // bins between exact re-anchorings
@@ -779,12 +783,13 @@ P5Choice p5_choice(bool stack, bool batch) {
   return c;
 }
 
-// angles per thread and groups per element pass for `na` angles
-P5Choice p5_pick(int na, bool stack, bool batch) {
+// Angles per thread and groups per element pass of a frame; of a batch, the angles of its class and
+// room for either number of groups.
+P5Choice p5_pick(int na, int groups, bool stack, bool batch) {
   if (na > 24) return p5_choice<8, 8>(stack, batch);
   if (na > 16) return p5_choice<6, 8>(stack, batch);
-  if (na > 8) return p5_choice<4, 12>(stack, batch);
-  return p5_choice<2, 12>(stack, batch);
+  if (na > 8) return groups > 8 ? p5_choice<4, 12>(stack, batch) : p5_choice<4, 8>(stack, batch);
+  return groups > 8 ? p5_choice<2, 12>(stack, batch) : p5_choice<2, 8>(stack, batch);
 }
 
 int p5_sms() {
@@ -803,8 +808,8 @@ cudaError_t p5_smem_optin() {
   std::lock_guard<std::mutex> lock(mu);
   if (dev < 64 && done[dev]) return cudaSuccess;
   for (int na : {8, 16, 24, 32})
-    for (int v = 0; v < 3; ++v) {
-      const P5Choice c = p5_pick(na, v == 1, v == 2);
+    for (int v = 0; v < 5; ++v) {
+      const P5Choice c = p5_pick(na, v < 3 ? 12 : 8, v == 1 || v == 4, v == 2);
       // the compute warps' register share needs the full allocation at launch
       cudaFuncAttributes a;
       if ((e = cudaFuncGetAttributes(&a, (const void*)c.fn)) != cudaSuccess) return e;
@@ -822,9 +827,9 @@ cudaError_t p5_smem_optin() {
 int pw_tc_class(int na) { return na > 16 ? 1 : 0; }
 
 size_t pw_tc_operand_bytes(int na, int K, int ne_pad) {
-  const P5Choice c = p5_pick(na, false, false);
+  const P5Choice c = p5_pick(na, 8, false, false);
   // a batch may run a frame with its class's widest passes
-  const P5Choice w = p5_pick(pw_tc_class(na) ? 32 : 16, false, false);
+  const P5Choice w = p5_pick(pw_tc_class(na) ? 32 : 16, 8, false, false);
   const size_t g = (size_t)K * (ne_pad >> 3) * 64;
   return std::max((size_t)((na + 4 * c.nt - 1) / (4 * c.nt)) * c.n, (size_t)((na + 4 * w.nt - 1) / (4 * w.nt)) * w.n) * g;
 }
@@ -862,7 +867,7 @@ cudaError_t launch_pw_tc_operand(const PWDev& d, int na_class, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(d.tc_max, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   pw_tc_absmax_kernel<<<304, 256, 0, s>>>(d, d.tc_max);
-  const P5Choice c = p5_pick(na_class > 0 ? na_class : d.na, false, false);
+  const P5Choice c = p5_pick(na_class > 0 ? na_class : d.na, 8, false, false);
   const int n_ap = (d.na + 4 * c.nt - 1) / (4 * c.nt);
   const size_t n = (size_t)n_ap * d.K * (d.ne_pad >> 3) * c.n * 2;
   pw_tc_operand_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, n_ap, c.nt, c.n);
@@ -873,7 +878,7 @@ cudaError_t launch_pw_tc(const PWDev& d0, bool stack, float2* image, float* weig
   cudaError_t e = p5_smem_optin();
   if (e == cudaSuccess) e = launch_pw_tc_operand(d0, 0, s);
   if (e != cudaSuccess) return e;
-  const P5Choice c = p5_pick(d0.na, stack, false);
+  const P5Choice c = p5_pick(d0.na, p5_groups(d0), stack, false);
   PWDev d = d0;
   const int slab = d0.wt_nc;
   for (int c0 = 0; c0 < d0.nx; c0 += slab) {
@@ -894,7 +899,7 @@ cudaError_t launch_pw_tc_batch(const PWBatchDev& B, int na_class, int grid, cuda
   cudaError_t e = p5_smem_optin();
   if (e == cudaSuccess) e = cudaMemsetAsync(B.counter, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  const P5Choice c = p5_pick(na_class, false, true);
+  const P5Choice c = p5_pick(na_class, 12, false, true);
   c.fn<<<grid, P5_THREADS, c.smem, s>>>(PWDev{}, nullptr, nullptr, B);
   return cudaGetLastError();
 }
