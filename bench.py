@@ -247,8 +247,10 @@ class Clocks:
         return {"sm_mhz": statistics.median(sm), "sm_max_mhz": mx, "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def pw_kernel_name(variant, window):
+def pw_kernel_name(variant, window, n_angles=11):
     """Name of the plane-wave fused kernel a plan's variant launches."""
+    if variant == 9 and n_angles <= 2:
+        return "pw_few_kernel<%d> (FP32; window %s from the plan's table)" % (n_angles, window)
     if variant == 9:
         return "pw_tc_kernel (tcgen05, fp16 hi/lo operands; window %s from the plan's table)" % window
     shapes = {1: (1, 11), 2: (2, 4), 3: (2, 2), 4: (4, 1)}
@@ -427,13 +429,13 @@ def run_ours(args):
     achieved = flops / (bf_avg_ms * 1e-3) / 1e12
     roof = {"bound": "fp32", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
             "frac": achieved / peak.value if peak.value else None, "traffic": traffic_from_profiles(info["kernel_variant"]) if args.kernel == "fused" else None,
-            "kernel": "pw_plain_kernel" if args.kernel == "plain" else pw_kernel_name(info["kernel_variant"], "hann"),
+            "kernel": "pw_plain_kernel" if args.kernel == "plain" else pw_kernel_name(info["kernel_variant"], "hann", len(wl.angles)),
             "work": "8 FLOP per active voxel x element x bin x angle term "
             "(complex MAC); %d active of %d nominal terms" % (info["active_terms"], info["terms"]),
             "executed_terms": info["executed_terms"],
             "peak_source": "measured FP32 FMA throughput (fnum_diag_fp32_peak); MEASURED_PEAKS.json "
             "holds only HBM and bf16 figures"}
-    if args.kernel == "fused" and info["kernel_variant"] == 9:
+    if args.kernel == "fused" and info["kernel_variant"] == 9 and len(wl.angles) > 2:
         # the tensor pipe: three products of 128 voxels x 8 complex elements x n columns per bin
         na = len(wl.angles)
         n = 16 if na <= 8 else (32 if na <= 16 else (48 if na <= 24 else 64))
@@ -465,8 +467,10 @@ def run_ours(args):
            "stage_ms": {"band_dft": float(np.mean(dft_ms)), "beamform": bf_avg_ms},
            "e2e": e2e, "roofline": roof, "cpu_baseline": cb, "clocks": clk, "accuracy": acc,
            # per step: the band DFT (operand split + tcgen05 GEMM) and the beamformer, which adds
-           # the scale and operand kernels for variant 9; no library kernels
-           "gpu_launches": args.steps * (5 if (args.kernel == "fused" and info["kernel_variant"] == 9) else 3),
+           # the scale and operand kernels for variant 9 (one or two angles: one kernel that
+           # lays the spectra out); no library kernels
+           "gpu_launches": args.steps * ((5 if len(wl.angles) > 2 else 4)
+                                         if (args.kernel == "fused" and info["kernel_variant"] == 9) else 3),
            "library_launches": {}}
     if anchor is not None:
         out["cfg1_anchor"] = anchor
@@ -696,10 +700,11 @@ def run_batch(args):
            "clocks": clk,
            # per frame: the band DFT (two kernels); a compounded tensor-core frame then its
            # scale and operand kernels, its tiles beamformed by the persistent launches (one
-           # per class of angle counts); other tensor-core frames add their own launch, FP32
+           # per class of angle counts); other frames of variant 9 add their own launch, FP32
            # frames one per image
            "gpu_launches": args.steps * (n_persist_launches + sum(
-               2 + ((2 if p.n_out == 1 else 3) if v == 9 else (1 if p.n_out == 1 else p.n_angles))
+               2 + ((2 if p.n_out == 1 or p.n_angles <= 2 else 3) if v == 9
+                    else (1 if p.n_out == 1 else p.n_angles))
                for p, v in zip(plans, variants)))}
     print(json.dumps(out))
     batch.close()

@@ -1656,10 +1656,11 @@ extern "C++" {
 namespace {
 
 // a frame that the persistent tensor-core launch can take: a compounded plane-wave plan
-// whose kernel variant is the tensor-core one
+// whose kernel variant is the tensor-core one, of more angles than launch_pw_few's
 bool tc_persistent(const fnum_plan* P) {
   return P->kind == 0 && P->n_out == 1 && !P->pw.m_sem && !(P->flags & FNUM_FLAG_PLAIN_KERNEL) &&
-         fnum::pw_variant_of(P->pw) == fnum::TC_VARIANT && P->pw.tc_B && P->pw.wt_nc == P->pw.nx;
+         fnum::pw_variant_of(P->pw) == fnum::TC_VARIANT && P->pw.na > 2 && P->pw.tc_B &&
+         P->pw.wt_nc == P->pw.nx;
 }
 
 template <typename T>

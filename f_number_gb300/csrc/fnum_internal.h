@@ -242,6 +242,9 @@ cudaError_t launch_pw_tc_operand(const PWDev& d, int widest, cudaStream_t s);
 // stack: one image per angle
 cudaError_t launch_pw_tc(const PWDev& d, bool stack, float2* image, float* weights, cudaStream_t s);
 cudaError_t launch_pw_tc_batch(const PWBatchDev& B, int widest, int grid, cudaStream_t s);
+// --- one or two angles (fnum_pw_few.cu) ---------------------------------------
+int pw_few_grid(const PWDev& d);
+cudaError_t launch_pw_few(const PWDev& d, bool stack, float2* image, float* weights, cudaStream_t s);
 cudaError_t launch_pw_plain(const PWDev& d, float2* image, float* weights, cudaStream_t s);
 constexpr int M_MAXE = 256;   // elements supported by the das_pw.m-semantics kernel
 cudaError_t launch_pw_m(const PWDev& d, int compound, float2* image, float* weights, cudaStream_t s);

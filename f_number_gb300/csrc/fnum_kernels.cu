@@ -1383,8 +1383,9 @@ static pw_kernel_t pw_pick_event_win(int window_id) {
 //     1: EPT 1 x NA 11   2: EPT 2 x NA 4   3: EPT 2 x NA 2   4: EPT 4 x NA 1
 //   boundaries resolved inside the bin loop (pw_fused_kernel):
 //     5: EPT 1 x NA 11   6: EPT 2 x NA 4   7: EPT 2 x NA 2   8: EPT 4 x NA 1
-//   9: tensor cores (fnum_pw_tc.cu), up to 32 angles per pass; needs the plan's
-//      operand scratch (PWDev::tc_B)
+//   9: tensor cores (fnum_pw_tc.cu), up to 32 angles per pass, or for one or two angles
+//      FP32 with the window table (fnum_pw_few.cu); needs the plan's operand scratch
+//      (PWDev::tc_B)
 // Angles beyond NA run as further passes inside the launch.  PWDev::variant
 // 0 picks by the angle count; a plan's autotuner may set another.
 static pw_kernel_t pw_variant_kernel(int v, const PWDev& d) {
@@ -1401,25 +1402,17 @@ static pw_kernel_t pw_variant_kernel(int v, const PWDev& d) {
   }
 }
 static int pw_fp32_variant(const PWDev& d) { return d.na >= 11 ? 1 : (d.na >= 4 ? 2 : (d.na >= 2 ? 3 : 4)); }
-// Default pass shape.  With the operand scratch in place the tensor cores take three angles
-// or more (11 angles of 128 elements on 512 x 512: 16.2 ms, the FP32 kernel 57 ms).  They run
-// one or two angles in the time of eight, the FP32 kernels in proportion, but on few tiles
-// those are bound by one tile's serial chain, which grows with the elements.  Measured,
-// FP32 | tensor cores, 2-7 MHz band:
-//   one angle, 128 elements: 24^2 5819 | 363 us, 256^2 4555 | 4175, 400^2 9141 | 9969
-//              64 elements:  24^2 2353 | 219,    128^2 1904 | 695,  400^2 3887 | 5061
-//   two angles, 128:         128^2 4700 | 1285,  400^2 13018 | 9973
-//               64:          128^2 2407 | 701,   400^2 5742 | 5064
-//               48:          128^2 1735 | 564,   400^2 4094 | 4097
-// so the crossing lies near 6 tiles (of 128 voxels) an element for one angle, and for two at
-// 64 elements.  Probes of up to 32 elements keep the FP32 kernel, which a batch runs beside
-// its persistent launches (24^2: 1229 | 151 us, 400^2: 1802 | 3131).
+// Default pass shape.  Variant 9 takes three angles or more on the tensor cores (11 angles of
+// 128 elements on 512 x 512: 15.9 ms, the FP32 kernel 57 ms) and fewer in FP32 with the window
+// table (fnum_pw_few.cu).  Measured, variant 4 or 3 | variant 9, 2-7 MHz band:
+//   one angle, 128 elements: 24^2 5806 | 300 us, 256^2 4555 | 1934, 400^2 9104 | 3979
+//              64 elements:  24^2 2346 | 176,    128^2 1902 | 423,  400^2 3930 | 2251
+//              32 elements:  24^2 1230 | 117,    400^2 1811 | 1417
+//   two angles, 128:         24^2 7336 | 394,    400^2 12909 | 6443
+// Probes of up to 32 elements keep the FP32 kernels for one or two angles (8 elements, 400^2:
+// 668 | 680 us), which a batch has always run beside its persistent launches.
 static int pw_default_variant(const PWDev& d) {
-  if (d.tc_B) {
-    if (d.na >= 3) return TC_VARIANT;
-    const long long tiles = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
-    if (d.ne > 32 && ((d.na == 2 && d.ne >= 64) || tiles <= 6ll * d.na * d.ne)) return TC_VARIANT;
-  }
+  if (d.tc_B && (d.na >= 3 || d.ne > 32)) return TC_VARIANT;
   return pw_fp32_variant(d);
 }
 static pw_kernel_t pw_pick(const PWDev& d) {
@@ -1537,8 +1530,8 @@ cudaError_t launch_pw_mma_deriv(const PWDev& d, int max_grid, float2* image, flo
 
 int pw_fused_grid(const PWDev& d, int* blocks_per_sm) {
   if (pw_variant_of(d) == TC_VARIANT) {
-    if (blocks_per_sm) *blocks_per_sm = 1;
-    return pw_tc_grid(d);
+    if (blocks_per_sm) *blocks_per_sm = d.na <= 2 ? 2 : 1;
+    return d.na <= 2 ? pw_few_grid(d) : pw_tc_grid(d);
   }
   pw_kernel_t fn = pw_pick(d);
   int dev = 0, nsm = 0, bps = 0;

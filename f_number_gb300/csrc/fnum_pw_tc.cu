@@ -875,6 +875,7 @@ cudaError_t launch_pw_tc_operand(const PWDev& d, int na_class, cudaStream_t s) {
 }
 
 cudaError_t launch_pw_tc(const PWDev& d0, bool stack, float2* image, float* weights, cudaStream_t s) {
+  if (d0.na <= 2) return launch_pw_few(d0, stack, image, weights, s);
   cudaError_t e = p5_smem_optin();
   if (e == cudaSuccess) e = launch_pw_tc_operand(d0, 0, s);
   if (e != cudaSuccess) return e;

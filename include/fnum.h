@@ -275,8 +275,8 @@ int fnum_das_pw_noalloc(const fnum_pw_desc* desc, const double* steering_angles,
    variant of a plane-wave plan on it (1: 1 element x 11 angles per pass,
    2: 2 x 4, 3: 2 x 2, 4: 4 x 1, with the segment boundaries resolved ahead of
    the bin loop; 5..8: the same shapes resolving them inside the bin loop;
-   9: tensor cores, up to 32 angles per pass, the default from 3 angles on and for
-   one or two angles of more than 32 elements unless the grid is large) at full
+   9: tensor cores, up to 32 angles per pass, and for one or two angles FP32 with
+   a window table; the default from 3 angles on and above 32 elements) at full
    occupancy, and keeps the fastest for the plan's later executes.  It allocates a temporary image and runs on
    a private stream (not capturable).  variant / ms (the chosen variant's
    beamform time) may be NULL.  A synthetic-aperture plan times its two
@@ -285,7 +285,7 @@ int fnum_das_pw_noalloc(const fnum_pw_desc* desc, const double* steering_angles,
    default when available); a FNUM_FLAG_PLAIN_KERNEL plan returns variant 0. */
 int fnum_plan_autotune(fnum_plan* plan, const void* d_rf, int rf_is_double, int* variant, float* ms);
 /* fnum_plan_set_kernel_variant: pins the fused-kernel variant of a plane-wave
-   plan (0 = by angles, elements and grid, 1..9 as above), e.g. one an earlier
+   plan (0 = by angles and elements, 1..9 as above), e.g. one an earlier
    fnum_plan_autotune chose.  Every variant gives the same images up to the
    rounding of the per-pass sums.  A synthetic-aperture plan accepts 0 (default),
    1 and 2 (when available); a plan with FNUM_FLAG_M_SEMANTICS or
@@ -310,7 +310,7 @@ int fnum_plan_set_shape(fnum_plan* plan, int blocks_per_sm, int bin_chunk);
    graph on `stream`; fnum_batch_frame_times gives, after it completed, each
    frame's completion time in ms from the batch's start (n values, in the
    order of `plans`). */
-/* Compounded frames whose plans use the tensor-core kernel (variant 9) are not
+/* Compounded frames of more than two angles that use variant 9 are not
    launched per frame: their band DFTs and spectra operands run on the branches,
    then ONE persistent launch per class of angle counts (up to 16, more)
    beamforms all of them -- each block

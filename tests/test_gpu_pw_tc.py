@@ -54,3 +54,14 @@ def test_image_matches_oracle(gpu, ne, na, nt, nx, nz, dx, win, compound):
     assert np.linalg.norm(img - o) <= TOL * np.linalg.norm(o)
     plan.close()
 
+
+
+@pytest.mark.parametrize("ne,na,nt,nx,nz,dx,win,compound", [
+    (2, 1, 300, 5, 33, 2.07e-4, windows.boxcar(), True),
+    (65, 1, 700, 4, 31, 1.513e-3, windows.hann(), True),             # two passes of 64 elements
+    (131, 2, 512, 6, 33, 4.03e-3, windows.tukey(0.5), True),
+    (40, 2, 384, 3, 20, 1.07e-3, windows.triangular(), False),
+])
+def test_few_angles_match_oracle(gpu, ne, na, nt, nx, nz, dx, win, compound):
+    """One and two angles (FP32 recurrences); the same bound, without the operand split."""
+    test_image_matches_oracle(gpu, ne, na, nt, nx, nz, dx, win, compound)
