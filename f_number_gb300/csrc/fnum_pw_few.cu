@@ -18,7 +18,8 @@
 // and 85 with 64.  One angle, 128 elements, 256 x 256: 4.55 ms with the segment-list kernel (its
 // weights change at nearly every bin, and a tile's boundaries are resolved serially), 4.13 ms on
 // the tensor cores, 2.05 ms here with chunks of 32 bins and 1.93 ms with 64.  Two blocks an SM:
-// three spill (2.19 ms).  One angle, 64 elements, 48 x 57: 1005, 185 and 132 us.
+// three spill (2.19 ms).  One angle, 64 elements, 48 x 57: 1005, 185 and 86 us (the
+// band in ranges of 16 bins).
 #include <cuda_runtime.h>
 #include <stdint.h>
 

@@ -848,11 +848,16 @@ int pw_tc_batch_grid() { return p5_sms(); }
 // Bin ranges per tile.  A tile is one block's work, so a frame of few tiles would leave most
 // SMs idle: its band is split into ranges of at least 64 bins (each pays two exact anchors and
 // the tile's set-up) until there are about six items per SM, so that the last wave costs a sixth.
+// The kernel for one or two angles has a shorter set-up: at least 32 bins, or 16 while 32 would
+// give fewer items than the 304 blocks that fit the SMs.  One angle, at least 64 | 32 | 16 bins:
+// 48 x 57 voxels, 64 elements 128 | 97 | 87 us, 64 x 64, 128 elements 483 | 317 | 299 us,
+// 128 x 128 581 | 580 | 599 us.
 void pw_tc_pick_split(PWDev& d) {
   const int tiles = ((d.nx + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
   int s = (6 * 152 + tiles - 1) / tiles;
-  s = std::max(1, std::min(s, d.K / 64));
-  d.split_bins = ((d.K + s - 1) / s + 31) / 32 * 32;
+  const int least = d.na > 2 ? 64 : (tiles * (d.K / 32) < 304 ? 16 : 32), unit = std::min(least, 32);
+  s = std::max(1, std::min(s, d.K / least));
+  d.split_bins = ((d.K + s - 1) / s + unit - 1) / unit * unit;
   d.split = (d.K + d.split_bins - 1) / d.split_bins;
 }
 
