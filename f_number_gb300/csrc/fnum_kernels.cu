@@ -785,7 +785,7 @@ pw_event_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ w
 // The differentiable binding's forward pass and dL/dc.  Its loss and dL/dc are FP64 values
 // that callers compare between versions to 1e-9, which fixes the rounding of every step
 // below them, so this path keeps its arithmetic; every other image comes from the kernel of
-// fnum_pw_tc.cu (150 x 203 voxels, 96 elements, 5 angles: 2.1 ms here, 1.2 ms there).
+// fnum_pw_tc.cu (150 x 203 voxels, 96 elements, 5 angles: 1.9 ms here, 1.1 ms there).
 //
 // Per bin k the compounded image gains
 //   sum_a t_{v,a}^k G_k(v, a),   G_k(v, a) = sum_e R_k(v, e) X_k(e, a),

@@ -399,7 +399,7 @@ int fnum_bmode(const void* d_image, long long n_voxels, int n_images, float floo
 int fnum_diag_fp32_peak(int device, double* tflops);
 /* Throughput of warp-level mma.sync m16n8k16 (fp16 operands, fp32
    accumulators) on `device`, TFLOP/s (2 x 16 x 8 x 16 per instruction): the
-   tensor-pipe denominator of the tensor-core plane-wave kernel (variant 9). */
+   tensor-pipe denominator of the mma.sync kernels (fnum_pw_forward). */
 int fnum_diag_mma_f16_peak(int device, double* tflops);
 
 #ifdef __cplusplus
