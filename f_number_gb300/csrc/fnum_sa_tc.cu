@@ -492,14 +492,15 @@ sa_tc_kernel(const SADev d, const uint4* __restrict__ Bt, const unsigned* __rest
           }
           const unsigned r = st_range(sh.rng[(ns + (uint32_t)s) % ST_NT][t]);
           if (b % 32 == 0) live = 0u;     // exact phasors
-          if (r == 0xffffffffu) {         // no aperture in the tile at this bin
-            live = 0u;
-            continue;
+          // Without an aperture in the tile the bin has no groups, and the one under way is
+          // finished below with its own phasors: the next one that has groups need not be its
+          // neighbour, so its head's phasors stepped back would be another bin's.
+          if (r != 0xffffffffu) {
+            te = sh.tab[(ns + (uint32_t)s) & 1u][t][vb];
+            g_lo = (int)(r & 0xffffu) >> 3;
+            g_hi = (0xffff - (int)(r >> 16)) >> 3;
+            mask = (2u << g_hi) - (1u << g_lo);
           }
-          te = sh.tab[(ns + (uint32_t)s) & 1u][t][vb];
-          g_lo = (int)(r & 0xffffu) >> 3;
-          g_hi = (0xffff - (int)(r >> 16)) >> 3;
-          mask = (2u << g_hi) - (1u << g_lo);
         }
         const bool wide = 16 * (g_hi - g_lo + 1) > ST_NARROW;
         const unsigned exact = mask & ~live;
