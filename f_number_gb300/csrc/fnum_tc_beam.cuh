@@ -22,23 +22,31 @@ static_assert(P5_M == 128, "a voxel per TMEM lane");
 // work before the wait (p5_ask) and the answer handed to the wait.
 __device__ __forceinline__ uint32_t p5_ask(uint32_t bar, uint32_t parity) { return mbar_test(bar, parity) ? 1u : 0u; }
 
-// Waits for the phase of parity `parity`.  After P5_SPIN failed tests (a fraction of a second at
-// the least) it gives up, records the timeout and tells the others, whose failing waits then
-// end at once: the work after it runs on stale data, ends, and the call reports the error.
-constexpr unsigned P5_SPIN = 1u << 22;
+// Waits for the phase of parity `parity`.  It gives up after WAIT_NS of the global timer (read every
+// P5_TESTS failed tests: a test may suspend the thread for a time of the hardware's choice, so a
+// count alone is no bound), records the timeout and tells the others, whose failing waits then end
+// at once; the work after it runs on stale data and ends.  The entry points that wait for the
+// device (the host-buffer calls, the gradients, fnum_plan_info_get) report the recorded timeout.
+constexpr unsigned P5_TESTS = 64;
+static_assert(WAIT_NS < (1ull << 32), "the lower half of the timer measures it");
 __device__ __forceinline__ bool p5_wait(uint32_t bar, uint32_t parity, uint32_t answer, volatile int* abort_flag,
                                         unsigned long long* err) {
   if (answer) return true;
-  uint32_t left;
+  uint32_t ok;
   asm volatile(
-      "{\n.reg .pred p, q;\n.reg .u32 f;\nmov.u32 %0, %3;\n"
+      "{\n.reg .pred p, q;\n.reg .u32 f, n, t0;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n@p bra P5_DONE;\n"
+      "mov.u32 t0, %globaltimer_lo;\n"
+      "P5_MORE:\nmov.u32 n, %3;\n"
       "P5_AGAIN:\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n@p bra P5_DONE;\n"
-      "ld.volatile.shared.u32 f, [%4];\nsub.u32 %0, %0, 1;\nsetp.ne.u32 q, f, 0;\nselp.u32 %0, 0, %0, q;\n"
-      "setp.ne.u32 q, %0, 0;\n@q bra P5_AGAIN;\nP5_DONE:\n}\n"
-      : "=&r"(left)
-      : "r"(bar), "r"(parity), "n"(P5_SPIN), "r"(smem_u32((const void*)abort_flag))
+      "ld.volatile.shared.u32 f, [%4];\nsetp.ne.u32 q, f, 0;\n@q bra P5_DONE;\n"
+      "sub.u32 n, n, 1;\nsetp.ne.u32 q, n, 0;\n@q bra P5_AGAIN;\n"
+      "mov.u32 f, %globaltimer_lo;\nsub.u32 f, f, t0;\nsetp.lt.u32 q, f, %5;\n@q bra P5_MORE;\n"
+      "P5_DONE:\nselp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "n"(P5_TESTS), "r"(smem_u32((const void*)abort_flag)), "n"((unsigned)WAIT_NS)
       : "memory");
-  if (left) return true;
+  if (ok) return true;
   *abort_flag = 1;
   atomicOr(err, ERR_TC_TIMEOUT);
   return false;

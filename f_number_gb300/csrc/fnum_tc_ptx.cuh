@@ -10,8 +10,8 @@
 namespace fnum {
 namespace tcx {
 
-// every wait on an mbarrier gives up after this long (the kernel then records an
-// error, frees its tensor memory and returns instead of spinning)
+// every wait on an mbarrier (mbar_wait, and p5_wait of the beamformers) gives up after this long:
+// the kernel then records an error, frees its tensor memory and returns instead of spinning
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
