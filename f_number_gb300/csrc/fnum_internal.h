@@ -167,6 +167,8 @@ struct PWBatchDev {
 constexpr unsigned long long ERR_SEG_OVERFLOW = 1ull;
 constexpr unsigned long long ERR_DFT_TIMEOUT = 2ull;   // a wait of the tensor-core DFT gave up
 constexpr unsigned long long ERR_TC_TIMEOUT = 4ull;    // a wait of a tcgen05 beamformer gave up
+// no error: the spectra of variant 9 hold a NaN or an infinity, which its operand leaves out (p5_nonfinite)
+constexpr unsigned long long FLAG_NONFINITE = 8ull;
 
 // Band DFT on the tensor cores (fnum_dft_tc.cu): RF lines split into fp16 hi/lo
 // planes a [2][nsig][Kp], twiddle planes b [2][Np][Kp], per-line scale; the TMA

@@ -47,8 +47,8 @@ struct FwShared {
 };
 constexpr int fw_smem(int na) { return ((int)sizeof(FwShared) + 127) / 128 * 128 + FW_BC * fw_ep(na) * na * 16; }
 
-// spectra as element pairs [bin][pair][angle] {Re, Re, Im, Im}, zero beyond the last element; and
-// no bin range of a tile is done yet
+// spectra as element pairs [bin][pair][angle] {Re, Re, Im, Im}, zero beyond the last element and for
+// values that are not finite; and no bin range of a tile is done yet
 __global__ void __launch_bounds__(256) fw_pairs_kernel(const PWDev d, float4* __restrict__ out) {
   const int np = d.ne_pad >> 1;
   const size_t n = (size_t)d.K * np * d.na;
@@ -66,6 +66,10 @@ __global__ void __launch_bounds__(256) fw_pairs_kernel(const PWDev d, float4* __
     for (int h = 0; h < 2; ++h) {
       const int e = 2 * p + h;
       x[h] = e < d.ne ? d.X[((size_t)e * d.K + kk) * d.x_na + d.x_a0 + a] : make_float2(0.0f, 0.0f);
+      if (!p5_finite(x[h])) {
+        x[h] = make_float2(0.0f, 0.0f);
+        atomicOr(&d.counters[2], FLAG_NONFINITE);
+      }
     }
     out[i] = make_float4(x[0].x, x[1].x, x[0].y, x[1].y);
   }
@@ -280,6 +284,8 @@ pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ wei
     for (int o = 0; o < NO; ++o)
       out[(size_t)o * nvox + vox] =
           make_float2((acc[o].x + sh.red[o][vb].x) * d.scale, (acc[o].y + sh.red[o][vb].y) * d.scale);
+    if (d.counters[2] & FLAG_NONFINITE)
+      p5_nonfinite(d, out + vox, STACK ? nvox : 0, cc, jc, kt, nb, 0, 1);
   }
   if (tid == 0) {
     atomicAdd(&d.counters[0], sh.n_active * (unsigned long long)NA);

@@ -632,6 +632,8 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
           out[vox] = make_float2(o.x * d.scale * inv_sigma, o.y * d.scale * inv_sigma);
         }
       }
+      if (valid && (STACK || slot == 0) && (d.counters[2] & FLAG_NONFINITE))
+        p5_nonfinite(d, out + vox, STACK ? nvox : 0, cc, jc, kt, nb, STACK ? slot : 0, STACK ? 4 : 1);
       if (d.split > 1) {
         // the last of the tile's bin ranges to finish adds them up, in order
         unsigned* cnt = &d.tile_cnt[(size_t)(d.wt_c0 / TILE_X) * ntz + tile];
@@ -712,14 +714,15 @@ __global__ void __launch_bounds__(128) pw_tc_window_kernel(const PWDev d, float*
   }
 }
 
-// largest |component| of the band spectra of the launch's angles (float bits; >= 0 floats order as ints)
+// largest |component| of the finite band spectra of the launch's angles (float bits; >= 0 floats
+// order as ints)
 __global__ void __launch_bounds__(256) pw_tc_absmax_kernel(const PWDev d, unsigned* out) {
   const size_t n = (size_t)d.ne * d.K * d.na;
   float m = 0.0f;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const size_t a = i % d.na, ek = i / d.na;
     const float2 x = d.X[ek * d.x_na + d.x_a0 + a];
-    m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
+    if (p5_finite(x)) m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
@@ -728,7 +731,7 @@ __global__ void __launch_bounds__(256) pw_tc_absmax_kernel(const PWDev d, unsign
 // B tiles of the spectra, in the order the products read them: [angle pass][bin][element
 // group of 8][hi, lo][8 columns n][K half][n][8 fp16].  Column n belongs to slot n / (N / 4);
 // with c = n % (N / 4), it holds the real (c % 4 < 2) or imaginary part of G for the slot's
-// angle j = 2 (c / 4) + c % 2.
+// angle j = 2 (c / 4) + c % 2.  Values that are not finite are left out (p5_nonfinite).
 __global__ void __launch_bounds__(256) pw_tc_operand_kernel(const PWDev d, int n_ap, int nt, int N) {
   const int G = d.ne_pad >> 3;
   const size_t n_all = (size_t)n_ap * d.K * G * N * 2;
@@ -754,6 +757,10 @@ __global__ void __launch_bounds__(256) pw_tc_operand_kernel(const PWDev d, int n
     const int e = 8 * g + 4 * kc + t;
     float2 x = make_float2(0.0f, 0.0f);
     if (j < nt && a < d.na && e < d.ne) x = d.X[((size_t)e * d.K + kk) * d.x_na + d.x_a0 + a];
+    if (!p5_finite(x)) {
+      x = make_float2(0.0f, 0.0f);
+      atomicOr(&d.counters[2], FLAG_NONFINITE);
+    }
     x.x *= sigma;
     x.y *= sigma;
     tc_split_mx(imag ? x.y : x.x, imag ? x.x : -x.y, h[t], l[t]);
