@@ -653,7 +653,7 @@ int setup_pw_tc(fnum_plan* P, int na, int n_img) {
   const size_t n_part = D.split > 1 ? (size_t)D.split * n_img * D.nx * D.nz : 0;
   // one allocation for all of it
   const size_t sizes[] = {col * D.wt_nc * sizeof(float), (size_t)(ne + 1) * D.wt_nc * sizeof(float), n_b, n_u,
-                          n_part * sizeof(float2), tiles * sizeof(unsigned), sizeof(unsigned)};
+                          n_part * sizeof(float2), tiles * sizeof(unsigned), na * sizeof(unsigned)};
   size_t off[8] = {0};
   for (int i = 0; i < 7; ++i) off[i + 1] = off[i] + (sizes[i] + 255) / 256 * 256;
   unsigned char* m = nullptr;
@@ -1806,7 +1806,7 @@ int fnum_batch_create(fnum_plan* const* plans, int n, const void* const* d_rf, c
       int widest = 1;
       for (const auto& G : B->groups)
         if (G.cls == fnum::pw_tc_class(plans[f]->pw.na)) widest = G.widest;
-      if (e == cudaSuccess) e = fnum::launch_pw_tc_operand(plans[f]->pw, widest, q);
+      if (e == cudaSuccess) e = fnum::launch_pw_tc_operand(plans[f]->pw, widest, false, q);
       if (e != cudaSuccess) s = cuda_status(e);
     }
     for (int i = 1; i < k && !s; ++i) {

@@ -75,7 +75,7 @@ struct PWDev {
   int4* seg;
   // tensor-core variant: spectra as B tiles of the products (pw_tc_operand_kernel; the mma.sync
   // kernel's fragments [angle pass][K][tc_S][tc_nt][32] share the buffer), and the largest
-  // |component| of the spectra (float bits) that sets their fp16 scale
+  // |component| of the spectra (float bits) that sets their fp16 scale: of all, or [na] of each angle
   uint4* tc_B;
   unsigned* tc_max;
   int tc_S;            // element groups of 8 in the fragments (TC_KS - 1 zero groups of padding included)
@@ -239,8 +239,8 @@ void pw_tc_pick_split(PWDev& d);
 // window table of the columns wt_c0 .. wt_c0 + wt_nc - 1
 cudaError_t launch_pw_tc_window(const PWDev& d, float* tab, float* sum, cudaStream_t s);
 // the spectra's scale and B tiles; widest: the largest angle count of the launch that reads
-// them (0: the frame's own)
-cudaError_t launch_pw_tc_operand(const PWDev& d, int widest, cudaStream_t s);
+// them (0: the frame's own); stack: a scale per angle
+cudaError_t launch_pw_tc_operand(const PWDev& d, int widest, bool stack, cudaStream_t s);
 // stack: one image per angle
 cudaError_t launch_pw_tc(const PWDev& d, bool stack, float2* image, float* weights, cudaStream_t s);
 cudaError_t launch_pw_tc_batch(const PWBatchDev& B, int widest, int grid, cudaStream_t s);

@@ -316,7 +316,7 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
       const unsigned un = p5_uni(p5_join(sh.un));
       const int E_lo = (int)(un & 0xffffu), E_hi = un == 0xffffffffu ? -1 : 0xffff - (int)(un >> 16);
       const int gp = p5_pass(BATCH ? min(p5_groups(d), GP) : GP, E_lo, E_hi);
-      const float inv_sigma = 1.0f / tc_scale(*d.tc_max);
+      const float inv_sigma = STACK ? 1.0f : 1.0f / tc_scale(*d.tc_max);
       const int n_grp = d.ne_pad >> 3;                      // element groups of 8 in the spectra
       const int tb = (d.tc_tb > 0 && d.tc_tb < 32) ? d.tc_tb : 32;   // bins between exact re-anchorings
       const int nstretch = (nb + P5_TT - 1) / P5_TT;
@@ -605,9 +605,10 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
               const int a = a0 + 4 * t + slot;
-              if (a < d.na)
-                out[(size_t)a * nvox + vox] =
-                    make_float2(sacc[t].x * d.scale * inv_sigma, sacc[t].y * d.scale * inv_sigma);
+              if (a < d.na) {
+                const float is = 1.0f / tc_scale(d.tc_max[a]);
+                out[(size_t)a * nvox + vox] = make_float2(sacc[t].x * d.scale * is, sacc[t].y * d.scale * is);
+              }
             }
           }
         }
@@ -714,25 +715,28 @@ __global__ void __launch_bounds__(128) pw_tc_window_kernel(const PWDev d, float*
   }
 }
 
-// largest |component| of the finite band spectra of the launch's angles (float bits; >= 0 floats
-// order as ints)
-__global__ void __launch_bounds__(256) pw_tc_absmax_kernel(const PWDev d, unsigned* out) {
-  const size_t n = (size_t)d.ne * d.K * d.na;
+// largest |component| of the finite band spectra (float bits; >= 0 floats order as ints): of all the
+// launch's angles into out[0], or with a row of blocks per angle (own) of each into out[angle]
+__global__ void __launch_bounds__(256) pw_tc_absmax_kernel(const PWDev d, unsigned* out, int own) {
+  const size_t na = own ? 1 : d.na, n = (size_t)d.ne * d.K * na;
   float m = 0.0f;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t a = i % d.na, ek = i / d.na;
+    const size_t ek = i / na, a = own ? blockIdx.y : i - ek * na;
     const float2 x = d.X[ek * d.x_na + d.x_a0 + a];
     if (p5_finite(x)) m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+  if ((threadIdx.x & 31) == 0) atomicMax(out + blockIdx.y, __float_as_uint(m));
 }
 
 // B tiles of the spectra, in the order the products read them: [angle pass][bin][element
 // group of 8][hi, lo][8 columns n][K half][n][8 fp16].  Column n belongs to slot n / (N / 4);
 // with c = n % (N / 4), it holds the real (c % 4 < 2) or imaginary part of G for the slot's
-// angle j = 2 (c / 4) + c % 2.  Values that are not finite are left out (p5_nonfinite).
-__global__ void __launch_bounds__(256) pw_tc_operand_kernel(const PWDev d, int n_ap, int nt, int N) {
+// angle j = 2 (c / 4) + c % 2.  Values that are not finite are left out (p5_nonfinite).  The fp16 scale
+// is common to the angles of a compound, whose products share an accumulator, and each angle's own
+// for images kept apart (own): what the loudest angle costs a quieter one in bits is lost in
+// their sum, but not in its own image.
+__global__ void __launch_bounds__(256) pw_tc_operand_kernel(const PWDev d, int n_ap, int nt, int N, int own) {
   const int G = d.ne_pad >> 3;
   const size_t n_all = (size_t)n_ap * d.K * G * N * 2;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -741,7 +745,6 @@ __global__ void __launch_bounds__(256) pw_tc_operand_kernel(const PWDev d, int n
     for (size_t t = i; t < n_tiles; t += (size_t)gridDim.x * blockDim.x) d.tile_cnt[t] = 0u;
   }
   if (i >= n_all) return;
-  const float sigma = tc_scale(*d.tc_max);
   const int in_group = (int)(i % (2 * N));
   size_t r = i / (2 * N);
   const int g = (int)(r % G);
@@ -751,6 +754,7 @@ __global__ void __launch_bounds__(256) pw_tc_operand_kernel(const PWDev d, int n
   const int slot = n / (N / 4), c = n % (N / 4);
   const int j = 2 * (c >> 2) + (c & 1), imag = (c >> 1) & 1;
   const int a = ap * 4 * nt + 4 * j + slot;
+  const float sigma = tc_scale(d.tc_max[own ? min(a, d.na - 1) : 0]);
   unsigned h[4], l[4];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
@@ -873,22 +877,23 @@ cudaError_t launch_pw_tc_window(const PWDev& d, float* tab, float* sum, cudaStre
   return cudaGetLastError();
 }
 
-cudaError_t launch_pw_tc_operand(const PWDev& d, int na_class, cudaStream_t s) {
+cudaError_t launch_pw_tc_operand(const PWDev& d, int na_class, bool stack, cudaStream_t s) {
   if (!d.tc_B || !d.tc_max) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(d.tc_max, 0, sizeof(unsigned), s);
+  const unsigned rows = stack ? (unsigned)d.na : 1u;
+  cudaError_t e = cudaMemsetAsync(d.tc_max, 0, rows * sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
-  pw_tc_absmax_kernel<<<304, 256, 0, s>>>(d, d.tc_max);
+  pw_tc_absmax_kernel<<<dim3((304 + rows - 1) / rows, rows), 256, 0, s>>>(d, d.tc_max, stack);
   const P5Choice c = p5_pick(na_class > 0 ? na_class : d.na, 8, false, false);
   const int n_ap = (d.na + 4 * c.nt - 1) / (4 * c.nt);
   const size_t n = (size_t)n_ap * d.K * (d.ne_pad >> 3) * c.n * 2;
-  pw_tc_operand_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, n_ap, c.nt, c.n);
+  pw_tc_operand_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, n_ap, c.nt, c.n, stack);
   return cudaGetLastError();
 }
 
 cudaError_t launch_pw_tc(const PWDev& d0, bool stack, float2* image, float* weights, cudaStream_t s) {
   if (d0.na <= 2) return launch_pw_few(d0, stack, image, weights, s);
   cudaError_t e = p5_smem_optin();
-  if (e == cudaSuccess) e = launch_pw_tc_operand(d0, 0, s);
+  if (e == cudaSuccess) e = launch_pw_tc_operand(d0, 0, stack, s);
   if (e != cudaSuccess) return e;
   const P5Choice c = p5_pick(d0.na, p5_groups(d0), stack, false);
   PWDev d = d0;
