@@ -684,13 +684,13 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
 // zero.  The half-width, and so the window, depends on the column and that element alone.
 __global__ void __launch_bounds__(128) pw_tc_window_kernel(const PWDev d, float* __restrict__ tab,
                                                            float* __restrict__ sum) {
-  const int col = d.wt_c0 + blockIdx.y, row = blockIdx.x, ne = d.ne;
+  const int col = d.wt_c0 + blockIdx.x, row = blockIdx.y, ne = d.ne;
   const dfl xm = d.col_m[col];
   const int emid = d.col_emid[col];
   const bool left = row < emid;
   float L = 0.0f;
   if (row < ne) L = left ? half_left(d.el_lb, xm, row, ne) : half_right(d.el_ub, xm, row);
-  float* o = tab + ((size_t)blockIdx.y * (ne + 1) + row) * d.ne_pad;
+  float* o = tab + ((size_t)blockIdx.x * (ne + 1) + row) * d.ne_pad;
   for (int e = threadIdx.x; e < d.ne_pad; e += blockDim.x) {
     float w = 0.0f;
     if (row < ne && L > 0.0f && (left ? (e >= row && e < emid) : (e >= emid && e <= row))) {
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(128) pw_tc_window_kernel(const PWDev d, float*
         W = win_sum_rt(d.window_id, (c.x - xm.x) + (c.y - xm.y), d.pitch_f, row - emid + 1, 1.0f / L, d.window_par, ip);
       }
     }
-    sum[(size_t)blockIdx.y * (ne + 1) + row] = W;
+    sum[(size_t)blockIdx.x * (ne + 1) + row] = W;
   }
 }
 
@@ -872,7 +872,7 @@ void pw_tc_pick_split(PWDev& d) {
 }
 
 cudaError_t launch_pw_tc_window(const PWDev& d, float* tab, float* sum, cudaStream_t s) {
-  const dim3 grid(d.ne + 1, d.wt_nc);
+  const dim3 grid(d.wt_nc, d.ne + 1);   // columns in x: y holds 65535 blocks, elements are 4096 at most
   pw_tc_window_kernel<<<grid, 128, 0, s>>>(d, tab, sum);
   return cudaGetLastError();
 }
