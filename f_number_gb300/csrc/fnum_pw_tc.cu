@@ -716,17 +716,17 @@ __global__ void __launch_bounds__(128) pw_tc_window_kernel(const PWDev d, float*
 }
 
 // largest |component| of the finite band spectra (float bits; >= 0 floats order as ints): of all the
-// launch's angles into out[0], or with a row of blocks per angle (own) of each into out[angle]
+// launch's angles into out[0], or with a column of blocks per angle (own) of each into out[angle]
 __global__ void __launch_bounds__(256) pw_tc_absmax_kernel(const PWDev d, unsigned* out, int own) {
   const size_t na = own ? 1 : d.na, n = (size_t)d.ne * d.K * na;
   float m = 0.0f;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t ek = i / na, a = own ? blockIdx.y : i - ek * na;
+  for (size_t i = (size_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.y * blockDim.x) {
+    const size_t ek = i / na, a = own ? blockIdx.x : i - ek * na;
     const float2 x = d.X[ek * d.x_na + d.x_a0 + a];
     if (p5_finite(x)) m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out + blockIdx.y, __float_as_uint(m));
+  if ((threadIdx.x & 31) == 0) atomicMax(out + blockIdx.x, __float_as_uint(m));
 }
 
 // B tiles of the spectra, in the order the products read them: [angle pass][bin][element
@@ -882,7 +882,7 @@ cudaError_t launch_pw_tc_operand(const PWDev& d, int na_class, bool stack, cudaS
   const unsigned rows = stack ? (unsigned)d.na : 1u;
   cudaError_t e = cudaMemsetAsync(d.tc_max, 0, rows * sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
-  pw_tc_absmax_kernel<<<dim3((304 + rows - 1) / rows, rows), 256, 0, s>>>(d, d.tc_max, stack);
+  pw_tc_absmax_kernel<<<dim3(rows, (304 + rows - 1) / rows), 256, 0, s>>>(d, d.tc_max, stack);
   const P5Choice c = p5_pick(na_class > 0 ? na_class : d.na, 8, false, false);
   const int n_ap = (d.na + 4 * c.nt - 1) / (4 * c.nt);
   const size_t n = (size_t)n_ap * d.K * (d.ne_pad >> 3) * c.n * 2;
