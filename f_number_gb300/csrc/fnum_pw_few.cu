@@ -11,19 +11,25 @@
 // threads form the window table's rows and n_k of every (bin, voxel) and the chunk's spectra are
 // copied to shared memory as element pairs {Re, Re, Im, Im}, the operands of packed FP32x2
 // instructions.  Then every warp takes its slot's groups of 8 elements within its column's
-// apertures, with the group's recurrences in registers.
+// apertures, with the group's recurrences in registers.  Where F is the same at all bins of a chunk
+// (constant, or at its bound) so are the apertures: the chunk then has one row per voxel and
+// its weights multiply the sums over the bins, not each term.
 //
-// What bounds it: issue slots (54 % busy) and the FMA pipe (54 %) at four warps a scheduler: about
-// 100 instructions per 8 elements and bin with chunks of 32 bins, of which 41 are the recurrence,
-// and 85 with 64.  One angle, 128 elements, 256 x 256: 4.55 ms with the segment-list kernel (its
-// weights change at nearly every bin, and a tile's boundaries are resolved serially), 4.13 ms on
-// the tensor cores, 2.05 ms here with chunks of 32 bins and 1.93 ms with 64.  Two blocks an SM:
-// three spill (2.19 ms).  One angle, 64 elements, 48 x 57: 1005, 185 and 86 us (the
-// band in ranges of 16 bins).
+// What bounds it: issue slots and the FMA pipe (54 % busy each where F varies) at four warps a
+// scheduler: about 100 instructions per 8 elements and bin with chunks of 32 bins, of which 41 are
+// the recurrence, and 85 with 64; chunks of one F need half of those.  One angle, 128 elements,
+// 256 x 256, F partly at its upper bound: 4.55 ms with the segment-list kernel (its weights change
+// at nearly every bin, and a tile's boundaries are resolved serially), 4.13 ms on the tensor cores,
+// 2.05 ms here with chunks of 32 bins, 1.93 ms with 64 and 1.67 ms with one weight for chunks of one F.
+// Constant F 1.5, 128 elements, 512 x 512, one | two angles: 2.23 | 3.72 ms with the segment-list
+// kernel (one segment a voxel), 2.71 | 4.32 ms with a weight a term, 1.43 | 2.75 ms with one a chunk.
+// Two blocks an SM: three spill (2.19 ms).  One angle, 64 elements, 48 x 57: 1005, 185 and 82 us
+// (the band in ranges of 16 bins).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "fnum_tc_beam.cuh"
 
@@ -118,11 +124,18 @@ pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ wei
       sh.lo[tid] = 0xffffu;
       sh.hi[tid] = -1;
     }
-    __syncthreads();
+    // one F for all the chunk's bins: one aperture and one weight per voxel and element
+    bool same = true;
+    if (tid < n) {
+      const dfl g0 = d.g[k_hi - d.k_lb], g1 = d.g[k_hi - tid - d.k_lb];
+      same = g0.x == g1.x && g0.y == g1.y;
+    }
+    const bool steady = __syncthreads_and(same);
     {
       unsigned lo = 0xffffu;
       int hi = -1;
-      for (int b = slot; b < n; b += 2) {
+      const int nt = steady ? 1 : n;             // table entries, each of n / nt bins
+      for (int b = slot; b < nt; b += 2) {
         const int kk = k_hi - b - d.k_lb;
         int ilb, iub;
         p5_aperture(xp, zp, d.g[kk], ne, ilb, iub);
@@ -132,7 +145,8 @@ pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ wei
         const int a = min(ilb, emid), z = max(iub, emid - 1);
         const bool act = valid && W > 0.0f && a <= z;
         if (valid) {
-          if (act) c_act += (unsigned)(z - a + 1); else ++c_emp;
+          const unsigned m = steady ? (unsigned)n : 1u;
+          if (act) c_act += m * (unsigned)(z - a + 1); else c_emp += m;
           if (kk == d.K - 1 && weights) weights[vox] = W;
         }
         sh.tab[b][vb] = make_uint2((unsigned)row_l | (unsigned)row_r << 16,
@@ -201,12 +215,8 @@ pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ wei
         const float4* xg = xs + (4 * g - p0) * NA;
         const uint2* tg = &sh.tab[0][vb];
         const float* wg = wcol + e8;
-#pragma unroll 1
-        for (int bs = 0; bs < n; bs += tb) {
-        const int be = min(bs + tb, n);
-#pragma unroll 4
-        for (int b = bs; b < be; ++b) {
-          const uint2 te = tg[b * P5_M];
+        // n_k w of the group's element pairs at table entry te
+        auto weigh = [&](uint2 te, float2 (&w)[4]) {
           const unsigned row = left ? te.x & 0xffffu : te.x >> 16;
           const float4* wr = reinterpret_cast<const float4*>(wg + row * (unsigned)d.ne_pad);
           float4 w0 = __ldg(wr), w1 = __ldg(wr + 1);
@@ -218,40 +228,64 @@ pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ wei
             w1 = make_float4(w1.x + z.x, w1.y + z.y, w1.z + z.z, w1.w + z.w);
           }
           const float2 nk = p5_dup(__uint_as_float(te.y));
-          const float2 w[4] = {__fmul2_rn(nk, make_float2(w0.x, w0.y)), __fmul2_rn(nk, make_float2(w0.z, w0.w)),
-                               __fmul2_rn(nk, make_float2(w1.x, w1.y)), __fmul2_rn(nk, make_float2(w1.z, w1.w))};
+          w[0] = __fmul2_rn(nk, make_float2(w0.x, w0.y));
+          w[1] = __fmul2_rn(nk, make_float2(w0.z, w0.w));
+          w[2] = __fmul2_rn(nk, make_float2(w1.x, w1.y));
+          w[3] = __fmul2_rn(nk, make_float2(w1.z, w1.w));
+        };
+        // the bins of the chunk; ONE: with the weights of a steady chunk after the sum
+        auto bins = [&](auto one) {
+          constexpr bool ONE = decltype(one)::value;
+          float2 w[4];
+          if constexpr (ONE) weigh(tg[0], w);
+#pragma unroll 1
+          for (int bs = 0; bs < n; bs += tb) {
+            const int be = min(bs + tb, n);
+#pragma unroll 4
+            for (int b = bs; b < be; ++b) {
+              if constexpr (!ONE) weigh(tg[b * P5_M], w);
 #pragma unroll
-          for (int x = 0; x < 4; ++x)
+              for (int x = 0; x < 4; ++x)
 #pragma unroll
-            for (int a = 0; a < NA; ++a) {
-              const float4 X = xg[b * (FW_EP * NA) + x * NA + a];
-              const float2 hr = Ar[a][x], hi = Ai[a][x];
-              Ar[a][x] = __ffma2_rn(hr, zr[a][x],
-                                    __ffma2_rn(hi, zn[a][x], __fmul2_rn(w[x], make_float2(X.x, X.y))));
-              Ai[a][x] = __ffma2_rn(hr, zi[a][x], __ffma2_rn(hi, zr[a][x], __fmul2_rn(w[x], make_float2(X.z, X.w))));
+                for (int a = 0; a < NA; ++a) {
+                  const float4 X = xg[b * (FW_EP * NA) + x * NA + a];
+                  float2 xr = make_float2(X.x, X.y), xi = make_float2(X.z, X.w);
+                  if constexpr (!ONE) {
+                    xr = __fmul2_rn(w[x], xr);
+                    xi = __fmul2_rn(w[x], xi);
+                  }
+                  const float2 hr = Ar[a][x], hi = Ai[a][x];
+                  Ar[a][x] = __ffma2_rn(hr, zr[a][x], __ffma2_rn(hi, zn[a][x], xr));
+                  Ai[a][x] = __ffma2_rn(hr, zi[a][x], __ffma2_rn(hi, zr[a][x], xi));
+                }
             }
-        }
-        // the exact phase at the stretch's last bin
-        const float kf = (float)(k_hi - be + 1);
+            // the exact phase at the stretch's last bin
+            const float kf = (float)(k_hi - be + 1);
 #pragma unroll
-        for (int x = 0; x < 4; ++x)
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
-          for (int a = 0; a < NA; ++a) {
-            dfl v0 = make_float2(uh[x].x, ul[x].x), v1 = make_float2(uh[x].y, ul[x].y);
-            if constexpr (NA > 1) {
-              v0 = df_add(v0, ua[a]);
-              v1 = df_add(v1, ua[a]);
-            }
-            float2 cr, ci;
-            p5_cis2(kf, make_float2(v0.x, v1.x), make_float2(v0.y, v1.y), cr, ci);
-            const float2 vr = __ffma2_rn(cr, Ar[a][x], p5_neg(__fmul2_rn(ci, Ai[a][x])));
-            const float2 vi = __ffma2_rn(cr, Ai[a][x], __fmul2_rn(ci, Ar[a][x]));
-            float2& s = sum[STACK ? a : 0];
-            s.x += vr.x + vr.y;
-            s.y += vi.x + vi.y;
-            Ar[a][x] = Ai[a][x] = make_float2(0.0f, 0.0f);
+              for (int a = 0; a < NA; ++a) {
+                dfl v0 = make_float2(uh[x].x, ul[x].x), v1 = make_float2(uh[x].y, ul[x].y);
+                if constexpr (NA > 1) {
+                  v0 = df_add(v0, ua[a]);
+                  v1 = df_add(v1, ua[a]);
+                }
+                float2 cr, ci;
+                p5_cis2(kf, make_float2(v0.x, v1.x), make_float2(v0.y, v1.y), cr, ci);
+                float2 vr = __ffma2_rn(cr, Ar[a][x], p5_neg(__fmul2_rn(ci, Ai[a][x])));
+                float2 vi = __ffma2_rn(cr, Ai[a][x], __fmul2_rn(ci, Ar[a][x]));
+                if constexpr (ONE) {
+                  vr = __fmul2_rn(w[x], vr);
+                  vi = __fmul2_rn(w[x], vi);
+                }
+                float2& s = sum[STACK ? a : 0];
+                s.x += vr.x + vr.y;
+                s.y += vi.x + vi.y;
+                Ar[a][x] = Ai[a][x] = make_float2(0.0f, 0.0f);
+              }
           }
-        }
+        };
+        if (steady) bins(std::true_type{}); else bins(std::false_type{});
         if (lane == 0) c_exec += (unsigned long long)(n * 8 * 32) * NA;
       }
 #pragma unroll
