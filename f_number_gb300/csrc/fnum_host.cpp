@@ -630,14 +630,53 @@ int pw_grid(const fnum_plan* P) {
   return fnum::pw_variant_of(P->pw) == fnum::TC_VARIANT ? g : std::min(g, P->max_grid);
 }
 
+// The elements that the window table holds for each column.  All of them while that takes no more
+// than 512 MB; for longer arrays those that the apertures of its tile's columns reach at the largest
+// depth and the band's smallest F, in 32s as the adjoint's warps take them (an element to spare for
+// the rounding of the aperture's ends): from e0, one for the tile, wt_w elements in wt_rows rows.
+// 4096 elements, F 1.5, 11 angles, 512 x 512: 34 GB and 112 ms refilled in turns of 4 columns, 0.1 GB
+// and 7.1 ms so.
+std::vector<int> window_band(fnum::PWDev& D, const double* px, const double* pz, double M, double pitch) {
+  const int nx = D.nx, ne = D.ne;
+  double z = 0.0;
+  for (int j = 0; j < D.nz; ++j) z = std::max(z, pz[j]);
+  const double half = D.gmax.x < 0.0f ? (double)ne : ((double)D.gmax.x + D.gmax.y) * z / pitch;
+  std::vector<int> e0(nx, 0);
+  int w = (size_t)(ne + 1) * D.ne_pad * nx * sizeof(float) <= (size_t)512 << 20 ? ne : 0;
+  for (int i = 0; i < nx && w < ne; i += fnum::TILE_X) {
+    const int end = std::min(i + fnum::TILE_X, nx);
+    double lo = ne - 1.0, hi = 0.0;
+    for (int c = i; c < end; ++c) {
+      const double p = M + px[c] / pitch;
+      lo = std::min(lo, floor(p - half) - 1.0);
+      hi = std::max(hi, ceil(p + half) + 1.0);
+    }
+    const int first = D.gmax.x < 0.0f ? 0 : (int)std::max(lo, 0.0) & ~31;
+    const int last = D.gmax.x < 0.0f ? ne - 1 : (int)std::min(hi, ne - 1.0);
+    for (int c = i; c < end; ++c) e0[c] = first;
+    w = std::max(w, last + 1 - first);
+  }
+  D.wt_w = (w + 31) / 32 * 32;
+  D.wt_rows = D.wt_w;
+  if (D.wt_w >= D.ne_pad) {
+    D.wt_w = D.ne_pad;
+    D.wt_rows = ne;
+    std::fill(e0.begin(), e0.end(), 0);
+  }
+  return e0;
+}
+
 // Tensor-core plane-wave kernel: window table, operand tiles and scratch.
-int setup_pw_tc(fnum_plan* P, int na, int n_img) {
+int setup_pw_tc(fnum_plan* P, int na, int n_img, const double* px, const double* pz, double M, double pitch) {
   fnum::PWDev& D = P->pw;
   const int ne = D.ne;
   D.ne_pad = (ne + 15) / 16 * 16;
-  // the table covers all columns, or as many as fit 512 MB (then it is refilled per launch)
-  const size_t col = (size_t)(ne + 1) * D.ne_pad;
-  const size_t fit = std::max<size_t>((((size_t)512 << 20) / (col * sizeof(float))) / 4 * 4, 4);
+  int* e0;
+  if (const int s = P->upload(&e0, window_band(D, px, pz, M, pitch))) return s;
+  D.col_e0 = e0;
+  // the table covers all columns, or as many as fit 4 GB (then it is refilled per launch)
+  const size_t col = (size_t)(D.wt_rows + 1) * D.wt_w;
+  const size_t fit = std::max<size_t>((((size_t)4 << 30) / (col * sizeof(float))) / 4 * 4, 4);
   D.wt_c0 = 0;
   D.wt_nc = (int)std::min<size_t>(fit, D.nx);
   fnum::pw_tc_pick_split(D);
@@ -652,7 +691,7 @@ int setup_pw_tc(fnum_plan* P, int na, int n_img) {
   const size_t n_u = fnum::pw_tc_scratch_bytes(fnum::pw_tc_grid(D));
   const size_t n_part = D.split > 1 ? (size_t)D.split * n_img * D.nx * D.nz : 0;
   // one allocation for all of it
-  const size_t sizes[] = {col * D.wt_nc * sizeof(float), (size_t)(ne + 1) * D.wt_nc * sizeof(float), n_b, n_u,
+  const size_t sizes[] = {col * D.wt_nc * sizeof(float), (size_t)(D.wt_rows + 1) * D.wt_nc * sizeof(float), n_b, n_u,
                           n_part * sizeof(float2), tiles * sizeof(unsigned), na * sizeof(unsigned)};
   size_t off[8] = {0};
   for (int i = 0; i < 7; ++i) off[i + 1] = off[i] + (sizes[i] + 255) / 256 * 256;
@@ -829,7 +868,8 @@ int make_pw_plan(const fnum_pw_desc* d, const double* angles, int na, int flags,
     D.seg = seg;
     P->info.scratch_bytes =
         (long long)P->max_grid * fnum::NTHREADS * D.seg_cap * fnum::PW_SEG_INT4 * (long long)sizeof(int4);
-    if ((s = setup_pw_tc(P, na, (flags & FNUM_FLAG_COMPOUND) ? 1 : na))) goto fail;
+    if ((s = setup_pw_tc(P, na, (flags & FNUM_FLAG_COMPOUND) ? 1 : na, d->positions_x, d->positions_z, b.M,
+                         d->element_pitch))) goto fail;
     // the default variant may now be the tensor-core one
     P->grid = pw_grid(P);
   }

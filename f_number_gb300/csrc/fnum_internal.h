@@ -81,12 +81,14 @@ struct PWDev {
   int tc_S;            // element groups of 8 in the fragments (TC_KS - 1 zero groups of padding included)
   int tc_nt;           // mma n-tiles per angle pass (3 or 4)
   // tensor-core kernel (fnum_pw_tc.cu): window table of columns wt_c0 .. wt_c0 + wt_nc - 1
-  // [column][ne + 1][ne_pad] and its row sums, the band's largest aperture, receive delays
-  // of the resident blocks, and for a band split into `split` ranges of split_bins bins
-  // their partial images and the finished ranges per tile
+  // [column][wt_rows + 1][wt_w] and its row sums: the elements from col_e0[column] (a tile's columns
+  // have one) that the band's largest aperture reaches, that aperture, receive delays of the
+  // resident blocks, and for a band split into `split` ranges of split_bins bins their partial
+  // images and the finished ranges per tile
   const float* w_tab;
   const float* w_sum;
-  int ne_pad, wt_c0, wt_nc;
+  const int* col_e0;
+  int ne_pad, wt_c0, wt_nc, wt_rows, wt_w;
   dfl gmax;
   float4* u_scr;
   int split, split_bins;

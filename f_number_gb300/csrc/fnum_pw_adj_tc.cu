@@ -90,9 +90,21 @@ __global__ void __launch_bounds__(256) aj_table_kernel(const PWDev d) {
   }
 }
 
+// whether the window table's elements of the columns of voxels v0 .. v1 - 1 reach elements e .. e + 127
+__device__ __forceinline__ bool aj_touched(const PWDev& d, long long v0, long long v1, int e) {
+  int lo = 0x7fffffff, hi = -1;
+  for (int i = ((int)(v0 / d.nz) & ~(TILE_X - 1)) + TILE_X * (int)(threadIdx.x & 31); i <= (int)((v1 - 1) / d.nz);
+       i += TILE_X * 32) {
+    lo = min(lo, d.col_e0[i]);
+    hi = max(hi, d.col_e0[i]);
+  }
+  return __reduce_min_sync(0xffffffffu, lo) < e + 128 && __reduce_max_sync(0xffffffffu, hi) + d.wt_w > e;
+}
+
 // N: D columns of a bin, two per angle.  [v_begin, v_end): the voxels of the window table's columns.  NB: bins of a
-// chunk (at most AJ_DCOLS / N).
-template <int N>
+// chunk (at most AJ_DCOLS / N).  BAND: the window table holds only the elements that the apertures reach;
+// items without any of them are passed over.
+template <int N, bool BAND>
 __global__ void __launch_bounds__(P5_THREADS, 1)
 aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __restrict__ gmax, double* __restrict__ acc,
              long long v_begin, long long v_end, int NB) {
@@ -143,12 +155,29 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
   uint32_t un = 0;                  // units (a group and a bin) of a slot so far
   uint32_t rd = 0;                  // rounds (groups of a slot) so far
   uint32_t it = 0;                  // items so far
+  // The block's items: every gridDim.x-th, with BAND of those that an aperture reaches (seen: such items
+  // of the slices and elements before `pair`), so that these are spread evenly over the blocks.
+  const int n_in = n_chunk * n_ap;
+  int next = blockIdx.x, seen = 0, pair = 0;
+  auto fetch = [&]() {
+    if constexpr (BAND) {
+      for (; pair < n_slice * n_ep; ++pair) {
+        const long long v0 = v_begin + (long long)(pair / n_ep) * AJ_SLICE;
+        if (!aj_touched(d, v0, min(v_end, v0 + AJ_SLICE), pair % n_ep * 128)) continue;
+        if (next < seen + n_in) return pair * n_in + next - seen;
+        seen += n_in;
+      }
+      return n_items;
+    } else {
+      return next;
+    }
+  };
 
   if (warp >= P5_CW) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P5_REGS_I));
     const uint32_t me = (uint32_t)(warp - P5_CW);       // issues the bins b % 4 = me of a chunk
     uint32_t ph2 = 0;                                   // phases of its s_full barriers (bit per round parity)
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    for (int item; (item = fetch()) < n_items; next += gridDim.x) {
       const int chunk = item % n_chunk;
       const int slice = item / (n_chunk * n_ap * n_ep);
       const int nb = min(NB, d.K - chunk * NB);
@@ -193,7 +222,7 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
     const float sigma = aj_scale(gmax);
     const int ne = d.ne;
     auto slot_bar = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + slot) : "memory"); };
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++it) {
+    for (int item; (item = fetch()) < n_items; next += gridDim.x) {
       const int chunk = item % n_chunk;
       int rest = item / n_chunk;
       const int a0 = (rest % n_ap) * NA;
@@ -224,11 +253,12 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
           int i, j;
           voxel(vv, i, j);
           const int kk = max(kt - b - d.k_lb, 0), cc = i - d.wt_c0, emid = d.col_emid[i];
+          const int e0 = BAND ? d.col_e0[i] : 0, zero = e0 + d.wt_rows;
           int ilb, iub;
           p5_aperture(d.col_p[i], d.row_p[j], d.g[kk], ne, ilb, iub);
           // a side without elements takes the zero row
-          const int row_l = ilb < emid ? ilb : ne, row_r = iub >= emid ? iub : ne;
-          const float* sc = d.w_sum + (size_t)cc * (size_t)(ne + 1);
+          const int row_l = ilb < emid ? ilb : zero, row_r = iub >= emid ? iub : zero;
+          const float* sc = d.w_sum + ((ptrdiff_t)cc * (d.wt_rows + 1) - e0);
           const float W = __ldg(sc + row_l) + __ldg(sc + row_r);
           const int lo = min(ilb, emid), hi = max(iub, emid - 1);
           const bool act = ok && W > 0.0f && lo <= hi;
@@ -239,22 +269,26 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
             mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
           }
           if (b < nb) {
-            const unsigned base = (unsigned)cc * (unsigned)(ne + 1);
+            // modulo 2^32: the element's number is added
+            const unsigned base = (unsigned)(cc * (d.wt_rows + 1) - e0), w = (unsigned)d.wt_w;
             sh.off[slot][buf][b][vv] =
-                make_uint2((base + (unsigned)row_l) * (unsigned)d.ne_pad, (base + (unsigned)row_r) * (unsigned)d.ne_pad);
+                make_uint2((base + (unsigned)row_l) * w - (unsigned)e0, (base + (unsigned)row_r) * w - (unsigned)e0);
             sh.nk[slot][buf][b][vv] = act ? (d.norm ? __frcp_rn(W) : 1.0f) : 0.0f;
             if (vv == 0) sh.rng[slot][buf][b] = (unsigned)mn | ((unsigned)(mx + 1) << 16);   // hi + 1: 0 for none
           }
         }
-        // the group's receive delays and steps, and on which side of the voxel the element lies
+        // the group's receive delays and steps, on which side of the voxel the element lies and, with BAND,
+        // whether the table holds it for the voxel's column: a group within one tile has all elements
+        // of a quadrant that an aperture touches
         float2 uh[4], ul[4];
         float rv[16];
-        unsigned left = 0u;
+        unsigned left = 0u, held = 0u;
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
           int i, j;
           voxel(x, i, j);
           if (e < d.col_emid[i]) left |= 1u << x;
+          if (BAND && (unsigned)(ec - d.col_e0[i]) < (unsigned)d.wt_w) held |= 1u << x;
           float4 t;
           if (d.rx_tab) {
             t = d.rx_tab[((size_t)i * d.nz + j) * ne + ec];
@@ -269,6 +303,7 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
           rv[4 * (x >> 1) + (x & 1)] = t.z;
           rv[4 * (x >> 1) + 2 + (x & 1)] = t.w;
         }
+        const bool whole = !BAND || __all_sync(0xffffffffu, held == 0xffu);
         slot_bar();     // rows and n_k of all the group's pairs
         // B: thread (voxel, angle) and, with 8 angles, half of the bins
         p5_wait(b_empty((uint32_t)slot, buf), ((rd >> 1) & 1u) ^ 1u, ask_b, abort_flag, err);
@@ -323,7 +358,8 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
               const uint2 of = sh.off[slot][buf][b][x];
-              w[x] = __ldg(d.w_tab + (((left >> x) & 1u ? of.x : of.y) + (unsigned)ec));
+              const unsigned o = ((left >> x) & 1u ? of.x : of.y) + (unsigned)ec;
+              w[x] = __ldg(d.w_tab + (whole || (held >> x) & 1u ? o : 0u));
             }
             if (live) {
               p5_rotate(p, rv);
@@ -338,6 +374,11 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
                 p[4 * x + 2] = im.x;
                 p[4 * x + 3] = im.y;
               }
+            }
+            if (BAND && !whole) {
+#pragma unroll
+              for (int x = 0; x < 8; ++x)
+                if (!((held >> x) & 1u)) w[x] = 0.0f;
             }
             p5_operand(make_float4(w[0], w[1], w[2], w[3]), make_float4(w[4], w[5], w[6], w[7]), p, h, l);
           } else {
@@ -384,6 +425,7 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
       }
       fence_before_sync();
       __syncthreads();
+      ++it;
     }
   }
   // after a timeout, give the products in flight time to land before the tensor memory is freed
@@ -431,7 +473,10 @@ cudaError_t launch_pw_adjoint(const PWDev& d0, const float2* cot, unsigned* gmax
                               cudaStream_t s) {
   const size_t n = (size_t)d0.ne * d0.K * d0.na;
   const int N = d0.na <= 8 ? 16 : 32;
-  const void* fn = N == 16 ? (const void*)aj_tc_kernel<16> : (const void*)aj_tc_kernel<32>;
+  const bool band = d0.wt_w < d0.ne_pad;
+  const auto kernel = N == 16 ? (band ? aj_tc_kernel<16, true> : aj_tc_kernel<16, false>)
+                              : (band ? aj_tc_kernel<32, true> : aj_tc_kernel<32, false>);
+  const void* fn = (const void*)kernel;
   // the compute warps' register share needs the full allocation at launch
   cudaFuncAttributes a;
   cudaError_t e = cudaFuncGetAttributes(&a, fn);
@@ -459,8 +504,7 @@ cudaError_t launch_pw_adjoint(const PWDev& d0, const float2* cot, unsigned* gmax
       return e;
     const long long v0 = (long long)c0 * d.nz, v1 = v0 + (long long)d.wt_nc * d.nz;
     const int nb = aj_bins(d, N, (int)((v1 - v0 + AJ_SLICE - 1) / AJ_SLICE), nsm);
-    if (N == 16) aj_tc_kernel<16><<<nsm, P5_THREADS, aj_smem(), s>>>(d, cot, gmax, acc, v0, v1, nb);
-    else aj_tc_kernel<32><<<nsm, P5_THREADS, aj_smem(), s>>>(d, cot, gmax, acc, v0, v1, nb);
+    kernel<<<nsm, P5_THREADS, aj_smem(), s>>>(d, cot, gmax, acc, v0, v1, nb);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   aj_finish_kernel<<<608, 256, 0, s>>>(acc, n, (double)d0.scale, gmax, gX);

@@ -105,8 +105,7 @@ pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ wei
   dfl ua[NA];
 #pragma unroll
   for (int a = 0; a < NA; ++a) ua[a] = df_add(d.tx_ax[(size_t)a * d.nx + ic], d.tx_az[(size_t)a * d.nz + jc]);
-  const float* wcol = d.w_tab + (size_t)cc * (size_t)(ne + 1) * d.ne_pad;
-  const float* wsum = d.w_sum + (size_t)cc * (size_t)(ne + 1);
+  const P5Window wt = p5_window(d, cc, (int)p5_uni((uint32_t)d.col_e0[ic]));
   const size_t nvox = (size_t)d.nx * d.nz, vox = (size_t)ic * d.nz + jc;
   const int tb = (d.tc_tb > 0 && d.tc_tb < 32) ? d.tc_tb : 32;   // bins between exact phases
   unsigned c_act = 0, c_emp = 0;
@@ -140,8 +139,8 @@ pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ wei
         int ilb, iub;
         p5_aperture(xp, zp, d.g[kk], ne, ilb, iub);
         // a side without elements takes the zero row
-        const int row_l = ilb < emid ? ilb : ne, row_r = iub >= emid ? iub : ne;
-        const float W = __ldg(wsum + row_l) + __ldg(wsum + row_r);
+        const int row_l = ilb < emid ? ilb : wt.zero, row_r = iub >= emid ? iub : wt.zero;
+        const float W = __ldg(wt.sum + row_l) + __ldg(wt.sum + row_r);
         const int a = min(ilb, emid), z = max(iub, emid - 1);
         const bool act = valid && W > 0.0f && a <= z;
         if (valid) {
@@ -214,15 +213,15 @@ pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ wei
         const bool left = e8 + 8 <= emid, mixed = e8 < emid && !left;
         const float4* xg = xs + (4 * g - p0) * NA;
         const uint2* tg = &sh.tab[0][vb];
-        const float* wg = wcol + e8;
+        const float* wg = wt.tab + e8;
         // n_k w of the group's element pairs at table entry te
         auto weigh = [&](uint2 te, float2 (&w)[4]) {
           const unsigned row = left ? te.x & 0xffffu : te.x >> 16;
-          const float4* wr = reinterpret_cast<const float4*>(wg + row * (unsigned)d.ne_pad);
+          const float4* wr = reinterpret_cast<const float4*>(wg + row * (unsigned)d.wt_w);
           float4 w0 = __ldg(wr), w1 = __ldg(wr + 1);
           if (mixed) {
             // the group around the voxel's column: the left side's values too
-            const float4* wl = reinterpret_cast<const float4*>(wg + (te.x & 0xffffu) * (unsigned)d.ne_pad);
+            const float4* wl = reinterpret_cast<const float4*>(wg + (te.x & 0xffffu) * (unsigned)d.wt_w);
             const float4 v = __ldg(wl), z = __ldg(wl + 1);
             w0 = make_float4(w0.x + v.x, w0.y + v.y, w0.z + v.z, w0.w + v.w);
             w1 = make_float4(w1.x + z.x, w1.y + z.y, w1.z + z.z, w1.w + z.w);

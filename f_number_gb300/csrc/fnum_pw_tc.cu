@@ -301,7 +301,7 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
       // this item's bins: kt down, nb of them
       const int kt = d.k_ub - part * d.split_bins;
       const int nb = min(d.split_bins, kt - d.k_lb + 1);
-      const int emid = (int)p5_uni((uint32_t)d.col_emid[ic]);
+      const int emid = (int)p5_uni((uint32_t)d.col_emid[ic]), e0 = (int)p5_uni((uint32_t)d.col_e0[ic]);
       if (slot == 0) {
         // the tile's elements: its apertures at the band's smallest F
         int ilb, iub;
@@ -343,7 +343,7 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
             const uint32_t tbuf = (ns + (uint32_t)s) & 1u, ri = (ns + (uint32_t)s) % P5_NT;
             const uint32_t ask = p5_ask(r_empty(ri), (((ns + (uint32_t)s) / P5_NT) & 1u) ^ 1u);
             const dfl xp = d.col_p[ic], zp = d.row_p[jc];
-            const float* sc = d.w_sum + (size_t)cc * (size_t)(ne + 1);
+            const P5Window wt = p5_window(d, cc, e0);
             int lo = 0xffff, hi = -1, rows[2];
             float inv[2];
 #pragma unroll
@@ -353,8 +353,8 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
               int ilb, iub;
               p5_aperture(xp, zp, d.g[kk], ne, ilb, iub);
               // a side without elements takes the zero row
-              const int row_l = ilb < emid ? ilb : ne, row_r = iub >= emid ? iub : ne;
-              const float W = __ldg(sc + row_l) + __ldg(sc + row_r);
+              const int row_l = ilb < emid ? ilb : wt.zero, row_r = iub >= emid ? iub : wt.zero;
+              const float W = __ldg(wt.sum + row_l) + __ldg(wt.sum + row_r);
               inv[t] = W > 0.0f ? (d.norm ? __frcp_rn(W) : 1.0f) : 0.0f;
               const int a = min(ilb, emid), z = max(iub, emid - 1);
               const bool act = valid && b < nb && W > 0.0f && a <= z;
@@ -362,7 +362,7 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
                 if (act) c_act += (unsigned)(z - a + 1); else ++c_emp;
                 if (kk == d.K - 1 && weights) weights[vox] = W;
               }
-              rows[t] = b < nb ? row_l | (row_r << 16) : ne | (ne << 16);   // beyond the band: weights 0
+              rows[t] = b < nb ? row_l | (row_r << 16) : wt.zero | (wt.zero << 16);   // beyond the band: weights 0
               if (act) {
                 lo = min(lo, a);
                 hi = max(hi, z);
@@ -377,7 +377,7 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
             mbar_arrive_if(lead, r_full(ri));
           };
           build(0);
-          const float* wcol = d.w_tab + (size_t)cc * (size_t)(ne + 1) * d.ne_pad + eb;
+          const float* wcol = p5_window(d, cc, e0).tab + eb;
           const int g_max = min(gp - 1, n_grp - 1 - (eb >> 3));
           // phasor steps rho = e^{2 pi i u} into shared memory, by element pairs {Re, Re, Im, Im};
           // the delays u to scratch for the exact anchors
@@ -506,8 +506,8 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
               const unsigned mask = g_lo <= g_hi ? (2u << g_hi) - (1u << g_lo) : 0u;
               const unsigned exact = mask & ~live;
               // rows of the window table (as offsets): left and right side of each bin
-              const unsigned ol0 = (unsigned)(te.x & 0xffff) * (unsigned)d.ne_pad, or0 = (unsigned)(te.x >> 16) * (unsigned)d.ne_pad;
-              const unsigned ol1 = (unsigned)(te.z & 0xffff) * (unsigned)d.ne_pad, or1 = (unsigned)(te.z >> 16) * (unsigned)d.ne_pad;
+              const unsigned ol0 = (unsigned)(te.x & 0xffff) * (unsigned)d.wt_w, or0 = (unsigned)(te.x >> 16) * (unsigned)d.wt_w;
+              const unsigned ol1 = (unsigned)(te.z & 0xffff) * (unsigned)d.wt_w, or1 = (unsigned)(te.z >> 16) * (unsigned)d.wt_w;
 #pragma unroll 1
               for (int g = g_lo + ((slot - g_lo) & 3); g <= g_hi; g += 4) {
                 const uint32_t tp = tl + (uint32_t)(C::PH + 16 * g);
@@ -678,26 +678,30 @@ pw_tc_kernel(const PWDev d0, float2* image0, float* weights0, const PWBatchDev B
 // ---------------------------------------------------------------------------
 // operands
 // ---------------------------------------------------------------------------
-// Window values w_tab[column][row][e] and their sums w_sum[column][row] of the slab's columns.
-// A row is the aperture's outermost element of one side: row r < emid holds the left side's
-// elements r .. emid - 1, row r >= emid the right side's emid .. r; row ne and the padding are
-// zero.  The half-width, and so the window, depends on the column and that element alone.
+// Window values w_tab[column][row][e] and their sums w_sum[column][row] of the slab's columns, rows and
+// elements counted from the column's first one e0.  A row is the aperture's outermost element of
+// one side: row r < emid holds the left side's elements r .. emid - 1, row r >= emid the right
+// side's emid .. r; the last row and the padding are zero.  The half-width, and so the window,
+// depends on the column and that element alone.
 __global__ void __launch_bounds__(128) pw_tc_window_kernel(const PWDev d, float* __restrict__ tab,
                                                            float* __restrict__ sum) {
-  const int col = d.wt_c0 + blockIdx.x, row = blockIdx.y, ne = d.ne;
+  const int col = d.wt_c0 + blockIdx.x, ne = d.ne, e0 = d.col_e0 ? d.col_e0[col] : 0;
+  const int row = (int)blockIdx.y < d.wt_rows ? e0 + (int)blockIdx.y : ne;
   const dfl xm = d.col_m[col];
   const int emid = d.col_emid[col];
   const bool left = row < emid;
   float L = 0.0f;
   if (row < ne) L = left ? half_left(d.el_lb, xm, row, ne) : half_right(d.el_ub, xm, row);
-  float* o = tab + ((size_t)blockIdx.x * (ne + 1) + row) * d.ne_pad;
-  for (int e = threadIdx.x; e < d.ne_pad; e += blockDim.x) {
+  const size_t line = (size_t)blockIdx.x * (d.wt_rows + 1) + blockIdx.y;
+  float* o = tab + line * d.wt_w;
+  for (int i = threadIdx.x; i < d.wt_w; i += blockDim.x) {
+    const int e = e0 + i;
     float w = 0.0f;
     if (row < ne && L > 0.0f && (left ? (e >= row && e < emid) : (e >= emid && e <= row))) {
       const dfl c = d.el_m[e];
       w = win_apply(d.window_id, d.window_par, fabsf((c.x - xm.x) + (c.y - xm.y)), L);
     }
-    o[e] = w;
+    o[i] = w;
   }
   if (threadIdx.x == 0) {
     float W = 0.0f;
@@ -711,7 +715,7 @@ __global__ void __launch_bounds__(128) pw_tc_window_kernel(const PWDev d, float*
         W = win_sum_rt(d.window_id, (c.x - xm.x) + (c.y - xm.y), d.pitch_f, row - emid + 1, 1.0f / L, d.window_par, ip);
       }
     }
-    sum[(size_t)blockIdx.x * (ne + 1) + row] = W;
+    sum[line] = W;
   }
 }
 
@@ -855,24 +859,24 @@ int pw_tc_items(const PWDev& d) {
 }
 int pw_tc_batch_grid() { return p5_sms(); }
 
-// Bin ranges per tile.  A tile is one block's work, so a frame of few tiles would leave most
+// Bin ranges per tile.  A tile is one block's work, so a launch of few tiles would leave most
 // SMs idle: its band is split into ranges of at least 64 bins (each pays two exact anchors and
 // the tile's set-up) until there are about six items per SM, so that the last wave costs a sixth.
 // The kernel for one or two angles has a shorter set-up: at least 32 bins, or 16 while 32 would
-// give fewer items than the 304 blocks that fit the SMs.  One angle, at least 64 | 32 | 16 bins:
+// give fewer items than the blocks that fit the SMs, two each.  One angle, at least 64 | 32 | 16 bins:
 // 48 x 57 voxels, 64 elements 128 | 97 | 87 us, 64 x 64, 128 elements 483 | 317 | 299 us,
 // 128 x 128 581 | 580 | 599 us.
 void pw_tc_pick_split(PWDev& d) {
-  const int tiles = ((d.nx + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
-  int s = (6 * 152 + tiles - 1) / tiles;
-  const int least = d.na > 2 ? 64 : (tiles * (d.K / 32) < 304 ? 16 : 32), unit = std::min(least, 32);
+  const int tiles = ((d.wt_nc + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z), nsm = p5_sms();
+  int s = (6 * nsm + tiles - 1) / tiles;
+  const int least = d.na > 2 ? 64 : (tiles * (d.K / 32) < 2 * nsm ? 16 : 32), unit = std::min(least, 32);
   s = std::max(1, std::min(s, d.K / least));
   d.split_bins = ((d.K + s - 1) / s + unit - 1) / unit * unit;
   d.split = (d.K + d.split_bins - 1) / d.split_bins;
 }
 
 cudaError_t launch_pw_tc_window(const PWDev& d, float* tab, float* sum, cudaStream_t s) {
-  const dim3 grid(d.wt_nc, d.ne + 1);   // columns in x: y holds 65535 blocks, elements are 4096 at most
+  const dim3 grid(d.wt_nc, d.wt_rows + 1);   // columns in x: y holds 65535 blocks, elements are 4096 at most
   pw_tc_window_kernel<<<grid, 128, 0, s>>>(d, tab, sum);
   return cudaGetLastError();
 }

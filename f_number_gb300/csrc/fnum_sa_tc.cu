@@ -742,7 +742,8 @@ int sa_tc_grid(const SADev& d) {
 cudaError_t launch_sa_tc_window(const SADev& d, cudaStream_t s) {
   PWDev w{};
   w.ne = d.ne;
-  w.ne_pad = d.ne_pad;
+  w.wt_rows = d.ne;
+  w.wt_w = d.ne_pad;
   w.wt_c0 = d.wt_c0;
   w.wt_nc = d.wt_nc;
   w.col_m = d.col_m;

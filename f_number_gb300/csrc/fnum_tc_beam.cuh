@@ -74,6 +74,19 @@ __device__ __forceinline__ void p5_aperture(dfl xp, dfl zp, dfl g, int ne, int& 
   aperture(xp, zp, g, ne, ilb, iub);
 }
 
+// A column's part of the window table: tab[row wt_w + e] and sum[row] by the numbers of the outermost
+// element (the row) and of the element, and the row of zeros.
+struct P5Window {
+  const float* tab;
+  const float* sum;
+  int zero;
+};
+__device__ __forceinline__ P5Window p5_window(const PWDev& d, int cc, int e0) {
+  const int rows = d.wt_rows + 1;
+  return {d.w_tab + ((ptrdiff_t)cc * rows * d.wt_w - (ptrdiff_t)e0 * (d.wt_w + 1)), d.w_sum + ((ptrdiff_t)cc * rows - e0),
+          e0 + d.wt_rows};
+}
+
 // Spectrum entries that are NaN or infinite stay out of the operands, where a weight of 0 (an
 // element of the same group outside the aperture) would turn them into NaN.  They are added to
 // the voxels whose aperture holds their element with a weight, whose values are then not finite
@@ -84,16 +97,15 @@ __device__ __forceinline__ bool p5_finite(float2 x) { return isfinite(x.x) && is
 [[maybe_unused]] static __device__ __noinline__ void p5_nonfinite(const PWDev& d, float2* out, size_t stride, int cc,
                                                                   int jc, int kt, int nb, int a0, int step) {
   const int ne = d.ne, ic = d.wt_c0 + cc, emid = d.col_emid[ic];
-  const float* wcol = d.w_tab + (size_t)cc * (size_t)(ne + 1) * d.ne_pad;
-  const float* wsum = d.w_sum + (size_t)cc * (size_t)(ne + 1);
+  const P5Window t = p5_window(d, cc, d.col_e0[ic]);
   for (int b = 0; b < nb; ++b) {
     const int kk = kt - b - d.k_lb;
     int ilb, iub;
     p5_aperture(d.col_p[ic], d.row_p[jc], d.g[kk], ne, ilb, iub);
-    const int row_l = ilb < emid ? ilb : ne, row_r = iub >= emid ? iub : ne;
-    if (!(wsum[row_l] + wsum[row_r] > 0.0f)) continue;
+    const int row_l = ilb < emid ? ilb : t.zero, row_r = iub >= emid ? iub : t.zero;
+    if (!(t.sum[row_l] + t.sum[row_r] > 0.0f)) continue;
     for (int e = min(ilb, emid); e <= max(iub, emid - 1); ++e) {
-      const float w = wcol[(size_t)(e < emid ? row_l : row_r) * d.ne_pad + e];
+      const float w = t.tab[(size_t)(e < emid ? row_l : row_r) * d.wt_w + e];
       if (!(w > 0.0f)) continue;
       for (int a = a0; a < d.na; a += step) {
         const float2 x = d.X[((size_t)e * d.K + kk) * d.x_na + d.x_a0 + a];
