@@ -630,8 +630,8 @@ int pw_grid(const fnum_plan* P) {
   return fnum::pw_variant_of(P->pw) == fnum::TC_VARIANT ? g : std::min(g, P->max_grid);
 }
 
-// The elements that the window table holds for each column.  All of them while that takes no more
-// than 512 MB; for longer arrays those that the apertures of its tile's columns reach at the largest
+// The elements that the window table holds for each column: all of up to 256 elements (263 KB a
+// column); of longer arrays those that the apertures of its tile's columns reach at the largest
 // depth and the band's smallest F, in 32s as the adjoint's warps take them (an element to spare for
 // the rounding of the aperture's ends): from e0, one for the tile, wt_w elements in wt_rows rows.
 // 4096 elements, F 1.5, 11 angles, 512 x 512: 34 GB and 112 ms refilled in turns of 4 columns, 0.1 GB
@@ -642,7 +642,7 @@ std::vector<int> window_band(fnum::PWDev& D, const double* px, const double* pz,
   for (int j = 0; j < D.nz; ++j) z = std::max(z, pz[j]);
   const double half = D.gmax.x < 0.0f ? (double)ne : ((double)D.gmax.x + D.gmax.y) * z / pitch;
   std::vector<int> e0(nx, 0);
-  int w = (size_t)(ne + 1) * D.ne_pad * nx * sizeof(float) <= (size_t)512 << 20 ? ne : 0;
+  int w = ne <= 256 ? ne : 0;
   for (int i = 0; i < nx && w < ne; i += fnum::TILE_X) {
     const int end = std::min(i + fnum::TILE_X, nx);
     double lo = ne - 1.0, hi = 0.0;

@@ -7,7 +7,7 @@
 // operands are split into fp16 hi + lo (Q scaled by a power of two) and hi.lo + lo.hi + hi.hi
 // accumulate in FP32 in tensor memory.  No counterpart in the reference.
 //
-// An item is a chunk of bins (their D's take up to 384 columns: 12 bins of 16 angles, 24 of 8), a
+// An item is a chunk of bins (their D's take up to 384 columns: 24 bins of 8 angles, 12 of 16, 8 of 24), a
 // slice of AJ_SLICE voxels, 128 elements and a pass of angles; the chunks of a slice run side by side,
 // so the receive table's rows come from L2.  16 warps form A: warp w serves lane quadrant w % 4
 // (an element per thread) and slot w / 4, which takes every fourth group of 8 voxels.  Per group
@@ -305,10 +305,11 @@ aj_tc_kernel(const PWDev d, const float2* __restrict__ cot, const unsigned* __re
         }
         const bool whole = !BAND || __all_sync(0xffffffffu, held == 0xffu);
         slot_bar();     // rows and n_k of all the group's pairs
-        // B: thread (voxel, angle) and, with 8 angles, half of the bins
+        // B: thread (voxel, angle) and, with 8 angles, half of the bins; the angles beyond 16 in a second turn
         p5_wait(b_empty((uint32_t)slot, buf), ((rd >> 1) & 1u) ^ 1u, ask_b, abort_flag, err);
-        {
-          const int vv = ts & 7, al = (ts >> 3) & (NA - 1), half = (NB + 1) / 2, b_lo = NA == 8 ? (ts >> 6) * half : 0;
+#pragma unroll 1
+        for (int al = (ts >> 3) & (NA == 8 ? 7 : 15); al < NA; al += 16) {
+          const int vv = ts & 7, half = (NB + 1) / 2, b_lo = NA == 8 ? (ts >> 6) * half : 0;
           const int b_hi = min(nb, NA == 8 ? b_lo + half : NB), a = a0 + al;
           const bool ok = vg + vv < v1 && a < d.na;
           const int ac = min(a, d.na - 1);
@@ -450,21 +451,31 @@ __global__ void __launch_bounds__(256) aj_finish_kernel(const double* __restrict
     gX[i] = make_float2((float)(sc * acc[2 * i]), (float)(sc * acc[2 * i + 1]));
 }
 
-// Bins per chunk: the most that D holds gives the fewest set-ups of a group (about as dear as
-// five bins), fewer give the SMs equal shares.
-int aj_bins(const PWDev& d, int N, int slices, int nsm) {
+// Bins per chunk of passes of N / 2 angles: the most that D holds gives the fewest set-ups of a
+// group (about as dear as five bins), fewer give the SMs equal shares.  cost: of the whole.
+int aj_bins(const PWDev& d, int N, int slices, int nsm, long long* cost) {
   const int per = slices * ((d.na + N / 2 - 1) / (N / 2)) * ((d.ne + 127) / 128);
   int best = AJ_DCOLS / N;
-  long long cost = 0;
+  *cost = 0;
   for (int nb = AJ_DCOLS / N; nb >= 4; --nb) {
     const long long items = (long long)((d.K + nb - 1) / nb) * per;
     const long long c = (items + nsm - 1) / nsm * (nb + 5);
-    if (cost == 0 || c < cost) {
-      cost = c;
+    if (*cost == 0 || c < *cost) {
+      *cost = c;
       best = nb;
     }
   }
   return best;
+}
+
+// D columns of a bin: passes of 8 angles, or of 16 or 24, whichever cost less (20 angles in passes of
+// 16 | 24: 128 elements, 400 x 300 voxels 11.5 | 7.1 ms, 64 x 64 0.77 | 0.80 ms).
+int aj_columns(const PWDev& d, int slices, int nsm) {
+  if (d.na <= 8) return 16;
+  long long c32, c48;
+  aj_bins(d, 32, slices, nsm, &c32);
+  aj_bins(d, 48, slices, nsm, &c48);
+  return c48 < c32 ? 48 : 32;
 }
 
 }  // namespace
@@ -472,10 +483,15 @@ int aj_bins(const PWDev& d, int N, int slices, int nsm) {
 cudaError_t launch_pw_adjoint(const PWDev& d0, const float2* cot, unsigned* gmax, float2* gX, double* acc,
                               cudaStream_t s) {
   const size_t n = (size_t)d0.ne * d0.K * d0.na;
-  const int N = d0.na <= 8 ? 16 : 32;
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  auto slices = [](long long v) { return (int)((v + AJ_SLICE - 1) / AJ_SLICE); };
+  const int N = aj_columns(d0, slices((long long)d0.wt_nc * d0.nz), nsm);
   const bool band = d0.wt_w < d0.ne_pad;
   const auto kernel = N == 16 ? (band ? aj_tc_kernel<16, true> : aj_tc_kernel<16, false>)
-                              : (band ? aj_tc_kernel<32, true> : aj_tc_kernel<32, false>);
+                    : N == 32 ? (band ? aj_tc_kernel<32, true> : aj_tc_kernel<32, false>)
+                              : (band ? aj_tc_kernel<48, true> : aj_tc_kernel<48, false>);
   const void* fn = (const void*)kernel;
   // the compute warps' register share needs the full allocation at launch
   cudaFuncAttributes a;
@@ -491,9 +507,6 @@ cudaError_t launch_pw_adjoint(const PWDev& d0, const float2* cot, unsigned* gmax
   if (e == cudaSuccess) e = launch_absmax(reinterpret_cast<const float*>(cot), 2 * (size_t)d0.nx * d0.nz, gmax, s);
   if (e != cudaSuccess) return e;
   if (d0.rx_tab) aj_table_kernel<<<1216, 256, 0, s>>>(d0);
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   PWDev d = d0;
   for (int c0 = 0; c0 < d0.nx; c0 += d0.wt_nc) {
     d.wt_c0 = c0;
@@ -503,7 +516,8 @@ cudaError_t launch_pw_adjoint(const PWDev& d0, const float2* cot, unsigned* gmax
                                 cudaSuccess)
       return e;
     const long long v0 = (long long)c0 * d.nz, v1 = v0 + (long long)d.wt_nc * d.nz;
-    const int nb = aj_bins(d, N, (int)((v1 - v0 + AJ_SLICE - 1) / AJ_SLICE), nsm);
+    long long cost;
+    const int nb = aj_bins(d, N, slices(v1 - v0), nsm, &cost);
     kernel<<<nsm, P5_THREADS, aj_smem(), s>>>(d, cot, gmax, acc, v0, v1, nb);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
