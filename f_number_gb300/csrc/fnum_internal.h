@@ -248,6 +248,7 @@ cudaError_t launch_pw_tc(const PWDev& d, bool stack, float2* image, float* weigh
 cudaError_t launch_pw_tc_batch(const PWBatchDev& B, int widest, int grid, cudaStream_t s);
 // --- one or two angles (fnum_pw_few.cu) ---------------------------------------
 int pw_few_grid(const PWDev& d);
+int pw_few_blocks(const PWDev& d);   // resident blocks per SM
 cudaError_t launch_pw_few(const PWDev& d, bool stack, float2* image, float* weights, cudaStream_t s);
 cudaError_t launch_pw_plain(const PWDev& d, float2* image, float* weights, cudaStream_t s);
 constexpr int M_MAXE = 256;   // elements supported by the das_pw.m-semantics kernel

@@ -1530,7 +1530,7 @@ cudaError_t launch_pw_mma_deriv(const PWDev& d, int max_grid, float2* image, flo
 
 int pw_fused_grid(const PWDev& d, int* blocks_per_sm) {
   if (pw_variant_of(d) == TC_VARIANT) {
-    if (blocks_per_sm) *blocks_per_sm = d.na <= 2 ? 2 : 1;
+    if (blocks_per_sm) *blocks_per_sm = d.na <= 2 ? pw_few_blocks(d) : 1;
     return d.na <= 2 ? pw_few_grid(d) : pw_tc_grid(d);
   }
   pw_kernel_t fn = pw_pick(d);

@@ -52,6 +52,9 @@ struct FwShared {
   int last;
 };
 constexpr int fw_smem(int na) { return ((int)sizeof(FwShared) + 127) / 128 * 128 + FW_BC * fw_ep(na) * na * 16; }
+constexpr int FW_BLOCKS = 2;             // resident per SM
+constexpr int FW_SMEM_ONE = 120 * 1024;  // more than half of an SM's shared memory: one resident block
+static_assert(fw_smem(1) <= FW_SMEM_ONE && fw_smem(2) <= FW_SMEM_ONE, "shared memory");
 
 // spectra as element pairs [bin][pair][angle] {Re, Re, Im, Im}, zero beyond the last element and for
 // values that are not finite; and no bin range of a tile is done yet
@@ -82,7 +85,7 @@ __global__ void __launch_bounds__(256) fw_pairs_kernel(const PWDev d, float4* __
 }
 
 template <int NA, bool STACK>
-__global__ void __launch_bounds__(FW_THREADS, 2)
+__global__ void __launch_bounds__(FW_THREADS, FW_BLOCKS)
 pw_few_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ weights) {
   extern __shared__ __align__(128) unsigned char dyn[];
   FwShared& sh = *reinterpret_cast<FwShared*>(dyn);
@@ -360,10 +363,13 @@ int pw_few_grid(const PWDev& d) {
   return ((d.wt_nc + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z) * d.split;
 }
 
+int pw_few_blocks(const PWDev& d) { return d.blocks_per_sm > 0 ? std::min(d.blocks_per_sm, FW_BLOCKS) : FW_BLOCKS; }
+
 cudaError_t launch_pw_few(const PWDev& d0, bool stack, float2* image, float* weights, cudaStream_t s) {
   if (!d0.tc_B || d0.na < 1 || d0.na > 2) return cudaErrorInvalidValue;
   const fw_kernel_t fn = fw_pick(d0.na, stack);
-  cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, fw_smem(d0.na));
+  const int smem = pw_few_blocks(d0) < FW_BLOCKS ? FW_SMEM_ONE : fw_smem(d0.na);
+  cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM_ONE);
   if (e != cudaSuccess) return e;
   fw_pairs_kernel<<<608, 256, 0, s>>>(d0, (float4*)d0.tc_B);
   PWDev d = d0;
@@ -374,7 +380,7 @@ cudaError_t launch_pw_few(const PWDev& d0, bool stack, float2* image, float* wei
     if (d0.wt_nc < d0.nx && (e = launch_pw_tc_window(d, const_cast<float*>(d.w_tab), const_cast<float*>(d.w_sum), s)) !=
                                 cudaSuccess)
       return e;
-    fn<<<pw_few_grid(d), FW_THREADS, fw_smem(d.na), s>>>(d, image, weights);
+    fn<<<pw_few_grid(d), FW_THREADS, smem, s>>>(d, image, weights);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   return cudaSuccess;

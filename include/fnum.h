@@ -292,7 +292,8 @@ int fnum_plan_autotune(fnum_plan* plan, const void* d_rf, int rf_is_double, int*
    FNUM_FLAG_PLAIN_KERNEL accepts only 0. */
 int fnum_plan_set_kernel_variant(fnum_plan* plan, int variant);
 /* fnum_plan_set_shape: pins the launch shape of a plane-wave plan's current
-   variant: blocks_per_sm (0 = as many as fit) and bin_chunk, the bins between
+   variant: blocks_per_sm, the most resident blocks of an SM (0 = as many as fit;
+   variant 9 has one from three angles on, else two), and bin_chunk, the bins between
    exact re-anchorings of the phase recurrences (0 = default; tensor cores 16 or
    32, FP32 kernels 128 or 256).  fnum_plan_autotune, after picking the variant,
    times these shapes (all or one fewer resident blocks, the default or the
