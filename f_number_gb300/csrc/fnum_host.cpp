@@ -2008,7 +2008,7 @@ int adjoint_core(fnum_plan* plan, const float2* G, float2* gX, double* dloss_dc,
   if (dloss_dc) FNUM_CUDA(cudaMemcpyAsync(&g, plan->adj_sums + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
   FNUM_CUDA(cudaMemcpyAsync(&err, plan->counters + 2, sizeof(err), cudaMemcpyDeviceToHost, st));
   FNUM_CUDA(cudaStreamSynchronize(st));
-  if (err & fnum::ERR_TC_TIMEOUT) return FNUM_ERR_INTERNAL;
+  if (err & (fnum::ERR_SEG_OVERFLOW | fnum::ERR_TC_TIMEOUT)) return FNUM_ERR_INTERNAL;
   if (dloss_dc) *dloss_dc = g;
   return FNUM_OK;
 }
@@ -2046,6 +2046,8 @@ int fnum_pw_adjoint(fnum_plan* plan, const void* d_cotangent, void* d_grad_spect
   int s;
   if ((s = fnum::adjoint_buffers(plan, st))) return s;
   float2* gX = d_grad_spectra ? (float2*)d_grad_spectra : plan->adj_gX;
+  // the error bits of this call alone (an earlier execute may have left some)
+  FNUM_CUDA(cudaMemsetAsync(plan->counters + 2, 0, sizeof(unsigned long long), st));
   return fnum::adjoint_core(plan, (const float2*)d_cotangent, gX, dloss_dc, false, st);
 }
 
