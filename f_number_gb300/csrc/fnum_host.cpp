@@ -666,37 +666,50 @@ std::vector<int> window_band(fnum::PWDev& D, const double* px, const double* pz,
   return e0;
 }
 
-// Tensor-core plane-wave kernel: window table, operand tiles and scratch.
-int setup_pw_tc(fnum_plan* P, int na, int n_img, const double* px, const double* pz, double M, double pitch) {
+// Variant 9 of a plane-wave plan: the layout of its window table, which covers all columns or as
+// many as fit 4 GB (then it is refilled per launch).
+int layout_pw_tc(fnum_plan* P, const double* px, const double* pz, double M, double pitch) {
   fnum::PWDev& D = P->pw;
-  const int ne = D.ne;
-  D.ne_pad = (ne + 15) / 16 * 16;
+  D.ne_pad = (D.ne + 15) / 16 * 16;
   int* e0;
   if (const int s = P->upload(&e0, window_band(D, px, pz, M, pitch))) return s;
   D.col_e0 = e0;
-  // the table covers all columns, or as many as fit 4 GB (then it is refilled per launch)
-  const size_t col = (size_t)(D.wt_rows + 1) * D.wt_w;
-  const size_t fit = std::max<size_t>((((size_t)4 << 30) / (col * sizeof(float))) / 4 * 4, 4);
+  const size_t col = (size_t)(D.wt_rows + 1) * D.wt_w * sizeof(float);
   D.wt_c0 = 0;
-  D.wt_nc = (int)std::min<size_t>(fit, D.nx);
+  D.wt_nc = (int)std::min<size_t>(std::max<size_t>(((size_t)4 << 30) / col / 4 * 4, 4), D.nx);
+  // the mma.sync kernels' fragments (32 uint4 per n-tile, bin and group of 8 elements)
+  D.tc_S = (D.ne + 7) / 8 + fnum::TC_KS - 1;
+  D.tc_nt = fnum::tc_ntiles_for(D.na);
   fnum::pw_tc_pick_split(D);
+  return FNUM_OK;
+}
+
+// Its memory: window table, operand tiles and scratch.  Where the device has no room for the table, it is
+// laid out for half of the columns, and again, down to a tile of them.
+int alloc_pw_tc(fnum_plan* P, cudaStream_t st) {
+  fnum::PWDev& D = P->pw;
+  const int na = D.na, n_img = (P->flags & FNUM_FLAG_COMPOUND) ? 1 : na;
+  const size_t col = (size_t)(D.wt_rows + 1) * D.wt_w;
   const size_t tiles = (size_t)((D.nx + fnum::TILE_X - 1) / fnum::TILE_X) * ((D.nz + fnum::TILE_Z - 1) / fnum::TILE_Z);
-  // the mma.sync kernels read the same buffer as fragments (32 uint4 per n-tile, bin and group of
-  // 8 elements; the derivative kernel in passes of 12 angles)
-  D.tc_S = (ne + 7) / 8 + fnum::TC_KS - 1;
-  D.tc_nt = fnum::tc_ntiles_for(na);
+  // the mma.sync kernels read the operand's buffer as fragments (the derivative kernel in passes of 12 angles)
   size_t n_b = fnum::pw_tc_operand_bytes(na, D.K, D.ne_pad);
   for (int nt : {3, D.tc_nt})
     n_b = std::max(n_b, (size_t)((na + 4 * nt - 1) / (4 * nt)) * D.K * D.tc_S * 32 * nt * sizeof(uint4));
-  const size_t n_u = fnum::pw_tc_scratch_bytes(fnum::pw_tc_grid(D));
-  const size_t n_part = D.split > 1 ? (size_t)D.split * n_img * D.nx * D.nz : 0;
-  // one allocation for all of it
-  const size_t sizes[] = {col * D.wt_nc * sizeof(float), (size_t)(D.wt_rows + 1) * D.wt_nc * sizeof(float), n_b, n_u,
-                          n_part * sizeof(float2), tiles * sizeof(unsigned), na * sizeof(unsigned)};
   size_t off[8] = {0};
-  for (int i = 0; i < 7; ++i) off[i + 1] = off[i] + (sizes[i] + 255) / 256 * 256;
   unsigned char* m = nullptr;
-  if (const int s = P->alloc(&m, off[7])) return s;
+  for (;;) {
+    const size_t n_u = fnum::pw_tc_scratch_bytes(fnum::pw_tc_grid(D));
+    const size_t n_part = D.split > 1 ? (size_t)D.split * n_img * D.nx * D.nz : 0;
+    // one allocation for all of it
+    const size_t sizes[] = {col * D.wt_nc * sizeof(float), (size_t)(D.wt_rows + 1) * D.wt_nc * sizeof(float), n_b, n_u,
+                            n_part * sizeof(float2), tiles * sizeof(unsigned), na * sizeof(unsigned)};
+    for (int i = 0; i < 7; ++i) off[i + 1] = off[i] + (sizes[i] + 255) / 256 * 256;
+    const int s = P->alloc(&m, off[7]);
+    if (s == FNUM_OK) break;
+    if (s != FNUM_ERR_OUT_OF_MEMORY || D.wt_nc <= fnum::TILE_X) return s;
+    D.wt_nc = std::max(D.wt_nc / 2 / fnum::TILE_X, 1) * fnum::TILE_X;
+    fnum::pw_tc_pick_split(D);
+  }
   float* tab = (float*)m;
   float* sum = (float*)(m + off[1]);
   D.w_tab = tab;
@@ -707,7 +720,7 @@ int setup_pw_tc(fnum_plan* P, int na, int n_img, const double* px, const double*
   D.tile_cnt = (unsigned*)(m + off[5]);
   D.tc_max = (unsigned*)(m + off[6]);
   P->info.scratch_bytes += (long long)off[7];
-  if (D.wt_nc == D.nx) FNUM_CUDA(fnum::launch_pw_tc_window(D, tab, sum, 0));
+  if (D.wt_nc == D.nx) FNUM_CUDA(fnum::launch_pw_tc_window(D, tab, sum, st));
   return FNUM_OK;
 }
 
@@ -868,8 +881,9 @@ int make_pw_plan(const fnum_pw_desc* d, const double* angles, int na, int flags,
     D.seg = seg;
     P->info.scratch_bytes =
         (long long)P->max_grid * fnum::NTHREADS * D.seg_cap * fnum::PW_SEG_INT4 * (long long)sizeof(int4);
-    if ((s = setup_pw_tc(P, na, (flags & FNUM_FLAG_COMPOUND) ? 1 : na, d->positions_x, d->positions_z, b.M,
-                         d->element_pitch))) goto fail;
+    if ((s = layout_pw_tc(P, d->positions_x, d->positions_z, b.M, d->element_pitch))) goto fail;
+    // a plan of the per-voxel kernel needs the memory for gradients alone (adjoint_buffers)
+    if (!(flags & FNUM_FLAG_PLAIN_KERNEL) && (s = alloc_pw_tc(P, 0))) goto fail;
     // the default variant may now be the tensor-core one
     P->grid = pw_grid(P);
   }
@@ -1495,7 +1509,7 @@ int fnum_plan_set_kernel_variant(fnum_plan* plan, int variant) {
     return FNUM_OK;
   }
   if (variant < 0 || variant > fnum::pw_variant_count()) return FNUM_ERR_ARGUMENT;
-  if (variant == fnum::TC_VARIANT && !plan->pw.tc_B) return FNUM_ERR_ARGUMENT;
+  if (variant == fnum::TC_VARIANT && !plan->pw.wt_nc) return FNUM_ERR_ARGUMENT;
   if (plan->pw.m_sem) return variant == 0 ? FNUM_OK : FNUM_ERR_ARGUMENT;     // one per-term kernel
   FNUM_CUDA(cudaSetDevice(plan->device));
   plan->pw.variant = variant;
@@ -1971,6 +1985,7 @@ int adjoint_buffers(fnum_plan* plan, cudaStream_t st) {
   const long long nvox = (long long)D.nx * D.nz;
   const size_t nspec = (size_t)D.ne * D.K * D.na;
   int s = FNUM_OK;
+  if (!D.tc_B && (s = fnum::alloc_pw_tc(plan, st))) return s;
   if (!plan->adj_img) {
     if ((s = plan->alloc(&plan->adj_img, (size_t)nvox)) || (s = plan->alloc(&plan->adj_G, (size_t)nvox)) ||
         (s = plan->alloc(&plan->adj_D, (size_t)nvox)) ||

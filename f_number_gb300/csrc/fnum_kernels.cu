@@ -1384,8 +1384,8 @@ static pw_kernel_t pw_pick_event_win(int window_id) {
 //   boundaries resolved inside the bin loop (pw_fused_kernel):
 //     5: EPT 1 x NA 11   6: EPT 2 x NA 4   7: EPT 2 x NA 2   8: EPT 4 x NA 1
 //   9: tensor cores (fnum_pw_tc.cu), up to 32 angles per pass, or for one or two angles
-//      FP32 with the window table (fnum_pw_few.cu); needs the plan's operand scratch
-//      (PWDev::tc_B)
+//      FP32 with the window table (fnum_pw_few.cu); needs a plan with a layout for that
+//      (PWDev::wt_nc)
 // Angles beyond NA run as further passes inside the launch.  PWDev::variant
 // 0 picks by the angle count; a plan's autotuner may set another.
 static pw_kernel_t pw_variant_kernel(int v, const PWDev& d) {
@@ -1412,7 +1412,7 @@ static int pw_fp32_variant(const PWDev& d) { return d.na >= 11 ? 1 : (d.na >= 4 
 // Probes of up to 32 elements keep the FP32 kernels for one or two angles (8 elements, 400^2:
 // 668 | 680 us), which a batch has always run beside its persistent launches.
 static int pw_default_variant(const PWDev& d) {
-  if (d.tc_B && (d.na >= 3 || d.ne > 32)) return TC_VARIANT;
+  if (d.wt_nc && (d.na >= 3 || d.ne > 32)) return TC_VARIANT;
   return pw_fp32_variant(d);
 }
 static pw_kernel_t pw_pick(const PWDev& d) {
@@ -1420,7 +1420,7 @@ static pw_kernel_t pw_pick(const PWDev& d) {
 }
 int pw_variant_count() { return 9; }
 int pw_mma_variant_of(const PWDev& d) {
-  return d.variant > 0 ? d.variant : (d.tc_B && d.na >= 3 ? TC_VARIANT : pw_fp32_variant(d));
+  return d.variant > 0 ? d.variant : (d.wt_nc && d.na >= 3 ? TC_VARIANT : pw_fp32_variant(d));
 }
 int pw_variant_of(const PWDev& d) { return d.variant > 0 ? d.variant : pw_default_variant(d); }
 
