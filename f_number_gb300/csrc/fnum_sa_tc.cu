@@ -707,12 +707,12 @@ size_t sa_tc_scratch_bytes(const SADev& d) {
   return (size_t)sa_tc_grid(d) * P5_M * 4 * ST_GMAX * sizeof(float4);
 }
 
-// Bin ranges per tile.  A tile is one block's work, so a frame of few tiles would leave SMs idle
+// Bin ranges per tile.  A tile is one block's work, so a launch of few tiles would leave SMs idle
 // in its last wave: its band is split into ranges of at least 64 bins (each pays the tile's
 // set-up) until there are about six items per SM.
 void sa_tc_pick_split(SADev& d) {
-  const int tiles = ((d.nx + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
-  int s = (6 * 152 + tiles - 1) / tiles;
+  const int tiles = ((d.wt_nc + TILE_X - 1) / TILE_X) * ((d.nz + TILE_Z - 1) / TILE_Z);
+  int s = (6 * st_sms() + tiles - 1) / tiles;
   s = std::max(1, std::min(s, d.K / 64));
   d.split_bins = ((d.K + s - 1) / s + 31) / 32 * 32;
   d.split = (d.K + d.split_bins - 1) / d.split_bins;
