@@ -24,7 +24,7 @@
 // serves lane quadrant w % 4 (a tile column, a voxel per thread) and element slot w / 4 (the
 // groups of 8 elements g with g % 4 = slot).  Per bin only the groups that the tile's apertures
 // touch run, with N = 16 (groups).  Per group a warp steps its phasors p <- p conj(rho) (kept in
-// tensor memory, 16 columns a group; exact every 32 bins and when a group comes back into
+// tensor memory, 16 columns a group; exact every 16 bins and when a group comes back into
 // range), multiplies them with the receive window and writes the split rows to its slot's A tile
 // in shared memory.  Two threads issue the group's products (each for half of the transmit
 // elements), two copy its B tiles in turn.  When a bin's D is complete every warp adds n_k sum_t w_tx p_t Y_t of its groups to its
@@ -66,6 +66,10 @@ using namespace tcx;
 
 constexpr int ST_GMAX = 16;                 // element groups of 8: up to 128 elements
 constexpr int ST_TT = 4;                    // bins per aperture table (one per slot)
+// Bins between exact phasors.  Error against 64 bits and time at 128 elements, 400 x 400, with 32 | 16 | 8:
+// 5.4e-7 | 4.3e-7 | 4.3e-7 and 18.70 | 18.84 | 19.09 ms; of nine other frames 4.0e-7 to 6.0e-7 with 32 (the
+// kernel before, whose products truncate less often, 3.7e-7 to 5.1e-7), 2.7e-7 to 4.9e-7 with 16.
+constexpr int ST_TB = 16;
 constexpr int ST_NT = 4;                    // element ranges in flight (aperture tables: 2)
 constexpr int ST_NB = 8;                    // B stages at most
 constexpr int ST_A = 2 * P5_M * 32;         // a slot's A tile: hi, lo
@@ -491,7 +495,7 @@ sa_tc_kernel(const SADev d, const uint4* __restrict__ Bt, const unsigned* __rest
             if (b + ST_TT < nb) build(s + 1);
           }
           const unsigned r = st_range(sh.rng[(ns + (uint32_t)s) % ST_NT][t]);
-          if (b % 32 == 0) live = 0u;     // exact phasors
+          if (b % ST_TB == 0) live = 0u;  // exact phasors
           // Without an aperture in the tile the bin has no groups, and the one under way is
           // finished below with its own phasors: the next one that has groups need not be its
           // neighbour, so its head's phasors stepped back would be another bin's.
