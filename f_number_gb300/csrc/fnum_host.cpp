@@ -2008,8 +2008,7 @@ int adjoint_buffers(fnum_plan* plan, cudaStream_t st) {
 
 // dL/dX* into gX and (if dloss_dc) dL/dc for the cotangent G = dL/dI*, on the plan's
 // spectra.  dL/dc needs the derivative image adj_D of those spectra: have_D says that the
-// caller has just computed it, else it is computed here (launch_pw_mma_deriv, whose
-// rounding goes with fnum_pw_forward's).
+// caller has just computed it, else it is computed here (launch_pw_mma_deriv).
 int adjoint_core(fnum_plan* plan, const float2* G, float2* gX, double* dloss_dc, bool have_D, cudaStream_t st) {
   fnum::PWDev& D = plan->pw;
   const long long nvox = (long long)D.nx * D.nz;

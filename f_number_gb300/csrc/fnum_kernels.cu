@@ -778,14 +778,12 @@ pw_event_kernel(const PWDev d, float2* __restrict__ image, float* __restrict__ w
 }
 
 // ---------------------------------------------------------------------------
-// plane-wave kernel on the tensor cores
-// ---------------------------------------------------------------------------
 // plane-wave image and derivative with warp-level mma.sync
 // ---------------------------------------------------------------------------
-// The differentiable binding's forward pass and dL/dc.  Its loss and dL/dc are FP64 values
-// that callers compare between versions to 1e-9, which fixes the rounding of every step
-// below them, so this path keeps its arithmetic; every other image comes from the kernel of
-// fnum_pw_tc.cu (150 x 203 voxels, 96 elements, 5 angles: 1.9 ms here, 1.1 ms there).
+// The differentiable binding's forward pass and dL/dc from three angles on; every other image
+// comes from the kernel of fnum_pw_tc.cu, which is faster (150 x 203 voxels, 96 elements, 5 angles:
+// 1.9 ms here, 1.1 ms there) and nearer to FP64 (4e-6 of the image here, 4e-7 there), but forms no
+// derivative: image and derivative are of one kernel, so that the gradient is that of the loss.
 //
 // Per bin k the compounded image gains
 //   sum_a t_{v,a}^k G_k(v, a),   G_k(v, a) = sum_e R_k(v, e) X_k(e, a),
@@ -1410,7 +1408,7 @@ static int pw_fp32_variant(const PWDev& d) { return d.na >= 11 ? 1 : (d.na >= 4 
 //              32 elements:  24^2 1230 | 117,    400^2 1811 | 1417
 //   two angles, 128:         24^2 7336 | 394,    400^2 12909 | 6443
 // Probes of up to 32 elements keep the FP32 kernels for one or two angles (8 elements, 400^2:
-// 668 | 680 us), which a batch has always run beside its persistent launches.
+// 668 | 680 us), although from 32 on variant 9 measured faster.
 static int pw_default_variant(const PWDev& d) {
   if (d.wt_nc && (d.na >= 3 || d.ne > 32)) return TC_VARIANT;
   return pw_fp32_variant(d);

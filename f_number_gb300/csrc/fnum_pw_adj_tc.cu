@@ -20,8 +20,8 @@
 // slice D is added to FP64 sums.
 //
 // The tensor cores' FP32 accumulation rounds toward zero, three times a group: 3.5e-5 of the
-// gradient (rel-L2) with slices of 8192 voxels, 8e-6 with 1024.  The longer slice is that of the
-// mma.sync kernel before this one, from whose gradients these stay within 2e-6.
+// gradient (rel-L2) with slices of 8192 voxels, as in the mma.sync kernel before this one (4e-5); with
+// 1024 it would be 8e-6.
 //
 // What bounds it: the compute warps' instructions, about 110 a unit (8 voxels x 32 elements x a
 // bin) and 600 a group for its set-up.  256 x 256 voxels, 128 elements, 11 angles: 12.9 ms with

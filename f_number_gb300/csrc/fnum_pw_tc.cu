@@ -29,8 +29,8 @@
 // cycles whatever its size, and an mbarrier answers a test after ~160, which set the two
 // issuers, the 8 x 2 unit (four products-worth a commit) and the tests asked ahead.
 // 11 angles, 128 elements, 512 x 512 voxels: 22.6 ms with warp-level mma.sync (window and
-// apertures re-formed per element pass, transmit recurrence per 16 elements), 15.9 ms here;
-// 31 angles, 192 elements, 301 x 451: 79.3 and 28.8 ms (fewer, wider angle passes); 11 images of
+// apertures re-formed per element pass, transmit recurrence per 16 elements), 16.0 ms here;
+// 31 angles, 192 elements, 301 x 451: 79.3 and 28.9 ms (fewer, wider angle passes); 11 images of
 // 161 x 224 kept apart: 47.7 and 2.5 ms (one launch instead of one FP32 launch per angle).
 #include <cuda.h>
 #include <cuda_fp16.h>

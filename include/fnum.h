@@ -367,11 +367,11 @@ int fnum_pw_sharpness_grad(fnum_plan* plan, const void* d_rf, int rf_is_double, 
    synchronises `stream`. */
 int fnum_pw_adjoint(fnum_plan* plan, const void* d_cotangent, void* d_grad_spectra, double* dloss_dc, void* stream);
 /* The image of a compounded plane-wave plan's current spectra (device float2
-   [n_x][n_z]) as the forward pass of a differentiable binding: the rounding of this
-   image, and with it that of FP64 losses formed from it and of fnum_pw_adjoint's
-   dL/dc, is kept between versions, so from three angles on it comes from an
-   mma.sync kernel where fnum_plan_execute_beamform runs variant 9 (equal up to
-   rounding).  No counterpart in the reference. */
+   [n_x][n_z]) as the forward pass of a differentiable binding.  From three angles
+   on it comes from the mma.sync kernel whose derivative pass gives
+   fnum_pw_adjoint's dL/dc (or from a pinned variant 1..8), not from variant 9 as
+   in fnum_plan_execute_beamform: within about 4e-6 (rel-L2) of the exact image,
+   where that is within 1e-6.  No counterpart in the reference. */
 int fnum_pw_forward(fnum_plan* plan, void* d_image, void* stream);
 /* loads band spectra (device float2, the layout of fnum_plan_spectra) into the
    plan, e.g. to beamform spectra a caller produced (fnum_plan_execute_beamform)
