@@ -258,9 +258,11 @@ def pw_kernel_name(variant, window, n_angles=11):
     return "%s<%d,%d,%s>" % ("pw_event_kernel" if variant <= 4 else "pw_fused_kernel", ept, na, window)
 
 
-def traffic_from_profiles(variant=9):
+def traffic_from_profiles(variant=9, n_angles=11):
     """DRAM bytes per launch of the launched kernel at the bench workload (ncu capture),
-    None for a variant without a capture."""
+    None for a variant or workload without a capture."""
+    if n_angles <= 2:
+        return None
     name = {9: "pw_tc_cpwc_512.json", 1: "pw_event_cpwc_512.json"}.get(variant)
     if name is None:
         return None
@@ -428,8 +430,8 @@ def run_ours(args):
     flops = 8.0 * info["active_terms"]
     achieved = flops / (bf_avg_ms * 1e-3) / 1e12
     roof = {"bound": "fp32", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
-            "frac": achieved / peak.value if peak.value else None, "traffic": traffic_from_profiles(info["kernel_variant"]) if args.kernel == "fused" else None,
-            "kernel": "pw_plain_kernel" if args.kernel == "plain" else pw_kernel_name(info["kernel_variant"], "hann", len(wl.angles)),
+            "frac": achieved / peak.value if peak.value else None, "traffic": traffic_from_profiles(info["kernel_variant"], wl.angles.size) if args.kernel == "fused" else None,
+            "kernel": "pw_plain_kernel" if args.kernel == "plain" else pw_kernel_name(info["kernel_variant"], win.spec()[0], len(wl.angles)),
             "work": "8 FLOP per active voxel x element x bin x angle term "
             "(complex MAC); %d active of %d nominal terms" % (info["active_terms"], info["terms"]),
             "executed_terms": info["executed_terms"],
@@ -759,7 +761,7 @@ def run_adjoint(args):
     b.record(stream)
     torch.cuda.synchronize()
     fwd_ms = a.elapsed_time(b)
-    # the adjoint alone (fnum_pw_adjoint without dL/dc: pw_adjoint_tc_kernel and its scale and finishing
+    # the adjoint alone (fnum_pw_adjoint without dL/dc: aj_tc_kernel and its scale and finishing
     # kernels), then with dL/dc (adds the derivative forward pass and its reduction), on the frame's spectra
     cot = torch.randn((plan.n_x, plan.n_z), dtype=torch.complex64, device=dev)
 
@@ -785,7 +787,7 @@ def run_adjoint(args):
     adj_tflops = 8.0 * info["active_terms"] / (adj_ms * 1e-3) / 1e12
     roof = {"bound": "fp32", "achieved": adj_tflops, "peak": peak.value, "unit": "TFLOP/s",
             "frac": adj_tflops / peak.value if peak.value else None, "traffic": None,
-            "kernel": "pw_adjoint_tc_kernel",
+            "kernel": "aj_tc_kernel",
             "work": "8 FLOP per active term (one complex MAC into dL/dX*, FP32-equivalent: the products run on "
                     "the tensor cores); %d active terms" % info["active_terms"],
             "peak_source": "measured FP32 FMA throughput (fnum_diag_fp32_peak)"}
