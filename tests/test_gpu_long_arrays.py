@@ -125,3 +125,28 @@ def test_adjoint_of_narrow_apertures(gpu, ne, na, nx, nz, dx):
         scale = (A.abs() * G.abs().double()).sum().item()
         assert abs(g[e, k, a].item() - want) <= tol * scale, (e, k, a)
     plan.close()
+
+
+def test_batch_with_a_table_in_turns(gpu):
+    """Such a frame keeps its own launches in a batch, beside the persistent ones: the images are those
+    of the plans by themselves, bit for bit."""
+    import torch
+    rng = np.random.default_rng(89)
+    plans = [_plan(NE, 3, 64, PX, PZ, windows.hann(), f_numbers.constant(0.0), FB)[2],
+             _plan(64, 5, 300, PX[:9], PZ, windows.hann(), f_numbers.constant(1.1), [3e6, 5e6])[2],
+             _plan(300, 3, 200, PX[:9], PZ, windows.boxcar(), f_numbers.constant(1.5), [3e6, 5e6])[2]]
+    rfs = [torch.tensor(rng.standard_normal(s), dtype=torch.float32, device=gpu)
+           for s in ((3, NE, 64), (5, 64, 300), (3, 300, 200))]
+    want = [p.execute(rf).clone() for p, rf in zip(plans, rfs)]
+    images = [torch.full_like(w, float("nan")) for w in want]
+    batch = das.Batch(plans, rfs, images, n_streams=2)
+    assert batch.persistent() == (2, 1)
+    for _ in range(2):
+        for im in images:
+            im.fill_(float("nan"))
+        batch.execute()
+        torch.cuda.synchronize()
+        assert all(torch.equal(im, w) for im, w in zip(images, want))
+    batch.close()
+    for p in plans:
+        p.close()
